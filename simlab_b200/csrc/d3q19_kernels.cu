@@ -22,6 +22,7 @@
 #include <utility>
 
 #include "lbm_device.cuh"
+#include "relax_fixed.cuh"
 #include "lbm_kernels.h"
 #include "tma.cuh"
 #include "reduce.cuh"
@@ -512,7 +513,11 @@ __global__ void __launch_bounds__(BLOCK) k_faces(const __grid_constant__ LatPara
 //
 // With NX * element size a multiple of 16 bytes and 512-byte aligned planes,
 // a shifted range's misalignment depends only on c_x, so each plane's first
-// cell sits at a compile-time element offset lead in its slot.  Store ranges
+// cell sits at a compile-time element offset lead in its slot.  For other row
+// lengths (RAG) the misalignment is still one number per plane, since tiles
+// start at whole units: it comes with the parameters, at one more addition per
+// access.  203 x 131 x 117 FP32: bulk 92 us per step with the direct kernel
+// (average of the parities), 80 staged; 301 x 157 x 157 BF16: 227 and 120.  Store ranges
 // are clamped to real cells and real slots, so no two blocks write the same
 // slot.  Requires non-periodic x and y; a periodic z wraps only at the z
 // boundaries, where cells load and store their wrapped links directly.
@@ -611,6 +616,16 @@ __global__ void k_wait_selftest(uint32_t *status, uint64_t limit_ns) {
     }
 }
 
+// the same for any row length: rows of whole 16-byte units leave only c_x in
+// a shift's misalignment; otherwise (RAG) parity 1 reads the plane's
+// misalignment, a constant of the lattice since tile starts are aligned, from
+// the parameters
+template <class S, int P, bool RAG>
+__device__ __forceinline__ uint32_t lead_of(const LatParams &p, int j) {
+    if constexpr (RAG && P == 1) return j == 0 ? 0u : p.lead[j];
+    else return (uint32_t)lead<S, P>(j);
+}
+
 // signed element shift of plane j's slots relative to the cell at parity P
 template <int P>
 __device__ __forceinline__ int64_t plane_shift(int j, int64_t NX, int64_t NXY) {
@@ -620,7 +635,7 @@ __device__ __forceinline__ int64_t plane_shift(int j, int64_t NX, int64_t NXY) {
 // The loads of tile n0 into a buffer by producer warp pw of NPROD: the
 // planes j = pw (mod NPROD), and the flags from the last producer; each
 // producer posts its own bytes on the buffer's "full" barrier.
-template <class S, int P, int NPROD>
+template <class S, int P, int NPROD, bool RAG>
 __device__ __forceinline__ void tma_load_tile(const LatParams &p, uint8_t *buf, uint64_t *bar, uint32_t n0, int pw) {
     constexpr uint32_t SLOT = slot_bytes<S>();
     constexpr uint32_t T = Tile<S>::cells;
@@ -631,7 +646,7 @@ __device__ __forceinline__ void tma_load_tile(const LatParams &p, uint8_t *buf, 
 #pragma unroll
     for (int j = 0; j < 19; j++) {
         if (j % NPROD != pw) continue;
-        const int64_t e = (int64_t)j * (int64_t)p.NP + n0 + plane_shift<P>(j, NX, NXY) - lead<S, P>(j);
+        const int64_t e = (int64_t)j * (int64_t)p.NP + n0 + plane_shift<P>(j, NX, NXY) - (int64_t)lead_of<S, P, RAG>(p, j);
         bulk_g2s(buf + j * SLOT, pop + e, SLOT, bar);
     }
     if (pw == NPROD - 1) bulk_g2s(buf + 19 * SLOT, p.flags + n0, T * 4, bar);
@@ -649,7 +664,7 @@ __host__ __device__ __forceinline__ constexpr int inward_dir(bool lo, int q) {
     return lo ? (q == 0 ? 1 : (q == 1 ? 7 : (q == 2 ? 9 : (q == 3 ? 13 : 15)))) : (q == 0 ? 2 : (q == 1 ? 8 : (q == 2 ? 10 : (q == 3 ? 14 : 16))));
 }
 
-template <class S, int P, bool LO>
+template <class S, int P, bool LO, bool RAG>
 __device__ __forceinline__ void xface_side(const LatParams &p, const StepParams &s, uint8_t *buf, uint32_t c, uint32_t m, uint32_t y,
                                            uint32_t z, const S *out) {
     using R = typename Pop<S>::real;
@@ -702,7 +717,7 @@ __device__ __forceinline__ void xface_side(const LatParams &p, const StepParams 
         if (!p.per[2] && (tz <= 0 || tz >= (int64_t)p.NZ - 1)) continue;
         const S v = Pop<S>::enc(fb[q], rng);
         const int j = P == 0 ? OPP(i) : i;
-        ((S *)(buf + j * SLOT))[lead<S, P>(j) + cb] = v;
+        ((S *)(buf + j * SLOT))[lead_of<S, P, RAG>(p, j) + cb] = v;
     }
 }
 
@@ -714,17 +729,17 @@ __device__ __forceinline__ void xface_side(const LatParams &p, const StepParams 
 // arithmetic and random sequence, and writes them into b's slots of the
 // staged tile; they reach HBM with the tile.  Only the 5 directions entering
 // the domain are needed (the face kernel's store mask of a planar x face).
-template <class S, int P>
+template <class S, int P, bool RAG>
 __device__ __forceinline__ void xface_from_inner(const LatParams &p, const StepParams &s, uint8_t *buf, uint32_t c, uint32_t m, uint32_t x,
                                                  uint32_t y, uint32_t z, const S *out) {
-    if (x == 1) xface_side<S, P, true>(p, s, buf, c, m, y, z, out);
-    else xface_side<S, P, false>(p, s, buf, c, m, y, z, out);
+    if (x == 1) xface_side<S, P, true, RAG>(p, s, buf, c, m, y, z, out);
+    else xface_side<S, P, false, RAG>(p, s, buf, c, m, y, z, out);
 }
 
 // A cell of a periodic-z boundary plane at input parity 1: the links that
 // leave the domain in z wrap to the other side, so those inputs and outputs go
 // straight to HBM; the others use the staged tile like every other cell.
-template <class S, int COLL>
+template <class S, int COLL, bool RAG>
 __device__ __forceinline__ void zwrap_cell(const LatParams &p, const StepParams &s, uint8_t *buf, uint32_t c, uint32_t n, uint32_t x,
                                         uint32_t y, uint32_t z) {
     using R = typename Pop<S>::real;
@@ -737,7 +752,7 @@ __device__ __forceinline__ void zwrap_cell(const LatParams &p, const StepParams 
     for (int i = 0; i < 19; i++) {
         const int j = i == 0 ? 0 : OPP(i);
         if (i > 0 && CZ(i) == -zw) f[i] = Pop<S>::ld(pop + (uint64_t)j * p.NP + (uint32_t)((int32_t)n + nb.off(-CX(i), -CY(i), -CZ(i))));
-        else f[i] = Pop<S>::cvt(((const S *)(buf + j * SLOT))[lead<S, 1>(j) + c]);
+        else f[i] = Pop<S>::cvt(((const S *)(buf + j * SLOT))[lead_of<S, 1, RAG>(p, j) + c]);
     }
     R rho, ux, uy, uz;
     const R om0[3] = {0, 0, 0};
@@ -747,11 +762,11 @@ __device__ __forceinline__ void zwrap_cell(const LatParams &p, const StepParams 
     for (int i = 0; i < 19; i++) {
         const S v = Pop<S>::enc(f[i], rng);
         if (i > 0 && CZ(i) == zw) pop[(uint64_t)i * p.NP + (uint32_t)((int32_t)n + nb.off(CX(i), CY(i), CZ(i)))] = v;
-        else ((S *)(buf + i * SLOT))[lead<S, 1>(i) + c] = v;
+        else ((S *)(buf + i * SLOT))[lead_of<S, 1, RAG>(p, i) + c] = v;
     }
 }
 
-template <class S, int P, int COLL, int FEAT>
+template <class S, int P, int COLL, int FEAT, bool RAG>
 __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tma(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
     using R = typename Pop<S>::real;
     constexpr int NBUF = Nbuf<S>::value;
@@ -776,7 +791,7 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
 #pragma unroll
         for (int j = 0; j < 19; j++) {
             tab_sh[j] = plane_shift<P>(j, (int64_t)p.NX, (int64_t)p.NX * p.NY);
-            tab_lead[j] = lead<S, P>(j);
+            tab_lead[j] = (int)lead_of<S, P, RAG>(p, j);
         }
     }
     __syncthreads();
@@ -823,7 +838,7 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
             }
             if (it < K && lane == 0) {
                 fence_async_smem();
-                tma_load_tile<S, P, NPROD>(p, sm + b * BUF, &full[b], (blockIdx.x + it * G) * T, pw);
+                tma_load_tile<S, P, NPROD, RAG>(p, sm + b * BUF, &full[b], (blockIdx.x + it * G) * T, pw);
             }
         }
         if (!alive && lane == 0) {
@@ -861,7 +876,7 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
             uint32_t x, y, z;
             coords(p, n, x, y, z);
             if (P == 1 && zper && (z == 0 || z == p.NZ - 1)) {
-                zwrap_cell<S, COLL>(p, s, buf, c, n, x, y, z);
+                zwrap_cell<S, COLL, RAG>(p, s, buf, c, n, x, y, z);
                 continue;
             }
             // FP16 values stay in storage units (x 32768) through the collision
@@ -870,13 +885,20 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
 #pragma unroll
             for (int i = 0; i < 19; i++) {
                 const int j = (P == 0 || i == 0) ? i : OPP(i);  // plane holding input f[i]
-                const S v = ((const S *)(buf + j * SLOT))[lead<S, P>(j) + c];
+                const S v = ((const S *)(buf + j * SLOT))[lead_of<S, P, RAG>(p, j) + c];
                 if constexpr (SC != 1) f[i] = __half2float(v);
                 else f[i] = Pop<S>::cvt(v);
             }
-            R rho, ux, uy, uz;
-            const R om0[3] = {0, 0, 0};
-            relax<R, COLL, SC, FEAT>(p, k, f, x, y, z, false, 0, 0, 0, 0, 0, om0, rho, ux, uy, uz);
+            if constexpr (RAG && FEAT != 0 && COLL == 0 && sizeof(R) == 4) {
+                // the direct kernel's roundings (its lattices' results stay
+                // what they were before they were staged)
+                const R sp = p.sponge_on ? sponge_at<R>(k, p, x, y, z) : (R)0;
+                relax_fixed<R, SC, (FEAT & 2) != 0, rf_direct<S, P>()>(k, moments<R>(f), sp, f);
+            } else {
+                R rho, ux, uy, uz;
+                const R om0[3] = {0, 0, 0};
+                relax<R, COLL, SC, FEAT>(p, k, f, x, y, z, false, 0, 0, 0, 0, 0, om0, rho, ux, uy, uz);
+            }
             Rng rng{sr_hash_mix(n, s.seed_mix)};
             S out[19];
             if constexpr (sizeof(S) == 2) {
@@ -885,12 +907,22 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
                 const uint32_t h = rng.s;
                 constexpr_for<0, 10>([&](auto kk) {
                     constexpr int K = decltype(kk)::value, i = 2 * K;
+                    // the bits of a ragged lattice are the direct kernel's: one
+                    // step of the sequence per value, of which the conversion
+                    // takes the upper half
+                    uint32_t bits;
+                    if constexpr (RAG) {
+                        const uint32_t b0 = rng.next();
+                        bits = i + 1 < 19 ? __byte_perm(b0, rng.next(), 0x7632) : b0;
+                    } else {
+                        bits = pair_bits<K>(h);
+                    }
                     if constexpr (i + 1 < 19) {
-                        const uint32_t h2 = Pop<S>::rs2(f[i + 1], f[i], pair_bits<K>(h));
+                        const uint32_t h2 = Pop<S>::rs2(f[i + 1], f[i], bits);
                         out[i] = Pop<S>::bits(h2 & 0xffffu);
                         out[i + 1] = Pop<S>::bits(h2 >> 16);
                     } else {
-                        out[i] = Pop<S>::bits(Pop<S>::rs2(f[i], 0.0f, pair_bits<K>(h)) >> 16);
+                        out[i] = Pop<S>::bits(Pop<S>::rs2(f[i], 0.0f, bits) >> 16);
                     }
                 });
             } else {
@@ -900,9 +932,9 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
 #pragma unroll
             for (int i = 0; i < 19; i++) {
                 const int j = (P == 0) ? OPP(i) : i;  // plane receiving output f[i]
-                ((S *)(buf + j * SLOT))[lead<S, P>(j) + c] = out[i];
+                ((S *)(buf + j * SLOT))[lead_of<S, P, RAG>(p, j) + c] = out[i];
             }
-            if (fg & FLAG_XFACE) xface_from_inner<S, P>(p, s, buf, c, n, x, y, z, out);
+            if (fg & FLAG_XFACE) xface_from_inner<S, P, RAG>(p, s, buf, c, n, x, y, z, out);
         }
         fence_async_smem();  // this thread's shared-memory writes, before the bulk stores read them
         mbar_arrive(&empty[b]);
@@ -1258,11 +1290,11 @@ static int num_sms() {
 }
 
 // persistent grid of the staged kernel: resident blocks per SM x SMs
-template <class S, int P, int COLL, int FEAT>
+template <class S, int P, int COLL, int FEAT, bool RAG>
 static unsigned tma_grid() {
     static unsigned g = 0;
     if (!g) {
-        auto kern = k_bulk_tma<S, P, COLL, FEAT>;
+        auto kern = k_bulk_tma<S, P, COLL, FEAT, RAG>;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_smem<S>());
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Tma<S>::threads, tma_smem<S>());
@@ -1271,10 +1303,28 @@ static unsigned tma_grid() {
     return g;
 }
 
+// RAG: rows that are no whole number of 16-byte units
 template <class S, int P, int COLL, int FEAT>
 static void launch_tma(const LatParams &p, const StepParams &s, cudaStream_t st) {
     const unsigned ntiles = (unsigned)((p.N + Tile<S>::cells - 1) / Tile<S>::cells);
-    k_bulk_tma<S, P, COLL, FEAT><<<std::min(ntiles, tma_grid<S, P, COLL, FEAT>()), Tma<S>::threads, tma_smem<S>(), st>>>(p, s);
+    // (ragged FP32, FP16 and BF16 lattices come here only with the regularized
+    // collision and compile-time features)
+    if constexpr (sizeof(S) == 8 || (COLL == 0 && FEAT != 0)) {
+        if (p.ragged) {
+            k_bulk_tma<S, P, COLL, FEAT, true><<<std::min(ntiles, tma_grid<S, P, COLL, FEAT, true>()), Tma<S>::threads, tma_smem<S>(), st>>>(p, s);
+            return;
+        }
+    }
+    k_bulk_tma<S, P, COLL, FEAT, false><<<std::min(ntiles, tma_grid<S, P, COLL, FEAT, false>()), Tma<S>::threads, tma_smem<S>(), st>>>(p, s);
+}
+
+uint32_t staged_tile_cells(int storage) {
+    switch (storage) {
+        case 0: return Tile<float>::cells;
+        case 1: return Tile<__half>::cells;
+        case 2: return Tile<__nv_bfloat16>::cells;
+        default: return Tile<double>::cells;
+    }
 }
 
 // one step: faces, wall cells (on the side stream `side` when they cannot
@@ -1302,6 +1352,7 @@ static cudaError_t step_t(const LatParams &p, const StepParams &s, cudaStream_t 
     if (overlap) cudaStreamWaitEvent(st, join, 0);
     else if (p.nrec) k_walls<S, P, COLL><<<(unsigned)((p.nrec + WBLOCK - 1) / WBLOCK), WBLOCK, 0, st>>>(p, s);
     if (ev && ev[2]) cudaEventRecord(ev[2], st);
+    // the staged kernel where it applies (lattice.cu, tma_ok), else the direct one
     if (p.tma) {
         if (!p.forcing && !p.abs_u) {
             if (p.les_on) launch_tma<S, P, COLL, 3>(p, s, st);

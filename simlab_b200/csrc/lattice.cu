@@ -387,11 +387,27 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
     // kernel while it collides m (flag bit FLAG_XFACE on m), one step ahead;
     // only the first step after setup or a state load needs the face kernel
     // for them.  They go to the end of the face list.
-    const bool tma_ok = (NX * storage_bytes(st.storage)) % 16 == 0 && !per[0] && !per[1];
+    const char *no_tma = std::getenv("SIMLAB_LBM_NO_TMA");
+    const bool ragged = (NX * storage_bytes(st.storage)) % 16 != 0;
+    const bool force = st.body_force[0] != 0.0 || st.body_force[1] != 0.0 || st.body_force[2] != 0.0;
+    // Rows that are no whole number of 16-byte units take the staged kernel's
+    // ragged variant where it rounds as the direct kernel does: the
+    // regularized collision without a body force, without the u_inf absorbing
+    // target and without periodic z (and FP64, whose roundings no result shows).
+    // Small lattices stay with it too: the staged kernel's few large tiles leave
+    // SMs idle.  Measured, us per step of a sphere in a tunnel, direct / staged:
+    // FP32 0.41 M cells 26.7 / 28.7, 0.82 M 36.0 / 36.8, 1.7 M 73.4 / 70.5, 3.6 M
+    // 134.6 / 122.3; FP16 28.2 / 31.3, 41.1 / 37.8, 67.0 / 52.0, 134.6 / 90.1
+    // (BF16 like FP16); FP64 27.6 / 27.6 at 0.1 M, 231 / 230 at 3.6 M.
+    const uint64_t ragged_from = st.storage == LBM_STORAGE_FP32 ? 1000000 : 640000;
+    const bool tma_ok = !per[0] && !per[1] && !(no_tma && no_tma[0] == '1') &&
+                        (!ragged || st.storage == LBM_STORAGE_FP64 ||
+                         (N >= ragged_from && st.collision == LBM_COLLISION_REGULARIZED && !force && !st.absorb_velocity && !per[2]));
+    const uint64_t tile = lbm::staged_tile_cells(st.storage);
     std::vector<char> fused(faces.size(), 0);
     uint32_t xinfo[2] = {0, 0};
     // (not with a spinning part, whose re-voxelizer rewrites the box flags)
-    if (tma_ok && !spin && !(std::getenv("SIMLAB_LBM_NO_TMA") && std::getenv("SIMLAB_LBM_NO_TMA")[0] == '1')) {
+    if (tma_ok && !spin && !ragged) {
         for (size_t k = 0; k < faces.size(); k++) {
             const uint64_t c = faces[k], x = c % NX, y = (c / NX) % NY, z = c / (NX * NY);
             if (x != 0 && x != NX - 1) continue;
@@ -400,6 +416,8 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
             if (y == 0 || y == NY - 1 || z == 0 || z == NZ - 1) continue;
             const uint64_t m = x == 0 ? c + 1 : c - 1;
             if (flags[m] != 0) continue;
+            // both in one staged tile (rows of odd length put some pairs across two)
+            if (c / tile != m / tile) continue;
             fused[k] = 1;
             flags[m] |= lbm::FLAG_XFACE;
             xinfo[x == 0 ? 0 : 1] = finfo[k] & 0xffu;
@@ -529,10 +547,16 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
     p.NX = (uint32_t)NX; p.NY = (uint32_t)NY; p.NZ = (uint32_t)NZ; p.N = (uint32_t)N;
     p.div_nx.init((uint32_t)NX);
     p.div_nxy.init((uint32_t)(NX * NY));
-    // the staged bulk kernel needs x-rows that keep 16-byte alignment and
-    // non-periodic x and y (its in-place tiles own their slots only then)
-    const char *no_tma = std::getenv("SIMLAB_LBM_NO_TMA");
-    p.tma = (NX * sb) % 16 == 0 && !per[0] && !per[1] && !(no_tma && no_tma[0] == '1');
+    // the staged bulk kernel needs non-periodic x and y (its in-place tiles
+    // own their slots only then); rows that are no whole number of 16-byte
+    // units take its variant with the planes' misalignments as parameters
+    p.tma = tma_ok;
+    p.ragged = ragged;
+    for (int j = 0; j < 19; j++) {
+        const int64_t unit = (int64_t)(16 / sb);
+        const int64_t shift = lbm::CX(j) + lbm::CY(j) * (int64_t)NX + lbm::CZ(j) * (int64_t)(NX * NY);
+        p.lead[j] = (uint32_t)((shift % unit + unit) % unit);
+    }
     p.nrec = (uint32_t)nrec; p.nface = (uint32_t)faces.size();
     for (int a = 0; a < 3; a++) p.per[a] = per[a];
     p.abs_u = st.absorb_velocity != 0;

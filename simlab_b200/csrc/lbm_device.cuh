@@ -147,7 +147,11 @@ struct LatParams {
     // the group's info (finfo[F]) instead of loading them.
     uint32_t frect[6], frect_b0[6], frect_sv[6], finfo[6];
     FastDiv frect_nu[6];
-    int tma;                   // the staged bulk kernel applies (NX * element size % 16 == 0)
+    int tma;                   // the staged bulk kernel applies (x and y not periodic)
+    int ragged;                // its rows are no whole number of 16-byte units
+    // ragged rows, parity 1: elements by which plane j's slots miss a 16-byte
+    // boundary at an aligned cell (c_j's shift modulo the unit)
+    uint32_t lead[19];
     // spinning part (Geometry::Spin, lattice.rs:87-92): every cell of the swept
     // box is a record, re-voxelized each step from the rotated surface
     const uint32_t *occ;       // body-frame occupancy bits on a fine grid

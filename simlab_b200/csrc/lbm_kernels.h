@@ -12,6 +12,8 @@ namespace lbm {
 // the step, after faces, after walls, after bulk
 cudaError_t launch_step(int storage, const LatParams &p, const StepParams &s, int parity, int coll, cudaStream_t st, cudaStream_t side,
                         cudaEvent_t fork, cudaEvent_t join, cudaEvent_t *ev = nullptr);
+// cells of one tile of the staged bulk kernel: tiles start at its multiples
+uint32_t staged_tile_cells(int storage);
 cudaError_t launch_init(int storage, const LatParams &p, cudaStream_t st);
 cudaError_t launch_dump(int storage, const LatParams &p, int q, cudaStream_t st);
 cudaError_t launch_sample(int storage, const LatParams &p, const StepParams &s, int q, const float *verts, uint32_t nvert, float voff,
