@@ -24,6 +24,7 @@
 #include "lbm_device.cuh"
 #include "relax_fixed.cuh"
 #include "lbm_kernels.h"
+#include "pdl.cuh"
 #include "tma.cuh"
 #include "reduce.cuh"
 #include "revoxel.cuh"
@@ -409,7 +410,7 @@ __device__ __forceinline__ void face_planar(const LatParams &p, const StepParams
 }
 
 template <class S, int P>
-__global__ void __launch_bounds__(BLOCK) k_faces(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
+__device__ __forceinline__ void faces_cell(const LatParams &p, const StepParams &s) {
     using R = typename Pop<S>::real;
     constexpr int Q = 1 - P;
     // the block's group: planar cells of one face (F < 6), or the rest
@@ -495,6 +496,18 @@ __global__ void __launch_bounds__(BLOCK) k_faces(const __grid_constant__ LatPara
         if (Q == 0 || i == 0) pop[(uint64_t)OPP(i) * p.NP + b] = v;
         else pop[(uint64_t)i * p.NP + (uint32_t)((int32_t)b + nb.off(CX(i), CY(i), CZ(i)))] = v;
     }
+}
+
+template <class S, int P>
+__global__ void __launch_bounds__(BLOCK) k_faces(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
+    pdl_release();
+    // beside the wall kernel (no wall cell near a face, so neither touches what
+    // the other does): the wall kernel let this one start after its own wait for
+    // the step before, and one thread's wait at the end keeps this grid from
+    // completing before the wall kernel has
+    if (!s.beside) pdl_wait();
+    faces_cell<S, P>(p, s);
+    if (s.beside && blockIdx.x == 0 && threadIdx.x == 0) pdl_wait();
 }
 
 // ---------------------------------------------------------------- staged bulk
@@ -795,6 +808,7 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
         }
     }
     __syncthreads();
+    pdl_wait();
     S *pop = (S *)p.pop;
     if (warp >= Tma<S>::cwarps) {
         constexpr int NPROD = Tma<S>::pwarps;
@@ -836,6 +850,10 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
                 }
                 __syncwarp();
             }
+            // the next kernel's blocks may come once every block is at its last
+            // tile: let in earlier, they all crowd onto the SMs whose blocks
+            // finish first (the 512x256x256 FP16 step 30 us longer)
+            if (it + 1 == K) pdl_release();
             if (it < K && lane == 0) {
                 fence_async_smem();
                 tma_load_tile<S, P, NPROD, RAG>(p, sm + b * BUF, &full[b], (blockIdx.x + it * G) * T, pw);
@@ -947,12 +965,6 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
 // bounce-back with the moving-wall term and Galilean-invariant momentum
 // exchange, shader.rs:399-436) and its post-collision state saved to the
 // record (437-441, 848-860).  Every record's F and T enter the step's sum.
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 static_assert((RS * 4) % 16 == 0, "records are read with 16-byte loads");
 // The record's first 32 words (mask, cell, q, post-collision populations)
 // in eight 16-byte loads.
@@ -1042,6 +1054,8 @@ __global__ void __launch_bounds__(WBLOCK) k_walls(const __grid_constant__ LatPar
     const Consts<R> &k = K<R>(p);
     const uint32_t r = blockIdx.x * WBLOCK + threadIdx.x;
     R Fo[3] = {0, 0, 0}, To[3] = {0, 0, 0};
+    pdl_wait();
+    pdl_release();
     if (r < p.nrec) {
         // The record's first 32 words, the cell's flag and its 19 populations
         // issued together before anything waits on them: the wall kernel is
@@ -1072,45 +1086,9 @@ __global__ void __launch_bounds__(WBLOCK) k_walls(const __grid_constant__ LatPar
             for (int a = 0; a < 3; a++) { Fo[a] = Rec<R>::ft(p, r, a); To[a] = Rec<R>::ft(p, r, 3 + a); }
         }
     }
-    // FP64 sum: warp shuffle -> block -> last block over all block partials
-    __shared__ double sh[WBLOCK / 32][6];
-    __shared__ bool last;
+    // FP64 sum: warp shuffle -> block partial (k_force_sum adds the blocks)
     double v[6] = {(double)Fo[0], (double)Fo[1], (double)Fo[2], (double)To[0], (double)To[1], (double)To[2]};
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int j = 0; j < 6; j++) v[j] = warp_sum(v[j]);
-    if (lane == 0)
-        for (int j = 0; j < 6; j++) sh[warp][j] = v[j];
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        double t = 0;
-        for (int w = 0; w < WBLOCK / 32; w++) t += sh[w][threadIdx.x];
-        p.partials[blockIdx.x * 8 + threadIdx.x] = t;
-        __threadfence();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t t = atomicAdd(p.ticket, 1u);
-        last = (t == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (uint32_t b = threadIdx.x; b < gridDim.x; b += WBLOCK)
-        for (int j = 0; j < 6; j++) acc[j] += __ldcg(&p.partials[b * 8 + j]);
-#pragma unroll
-    for (int j = 0; j < 6; j++) acc[j] = warp_sum(acc[j]);
-    __syncthreads();
-    if (lane == 0)
-        for (int j = 0; j < 6; j++) sh[warp][j] = acc[j];
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        double t = 0;
-        for (int w = 0; w < WBLOCK / 32; w++) t += sh[w][threadIdx.x];
-        p.hist[s.slot * 8 + threadIdx.x] = t;
-    }
-    if (threadIdx.x == 0) *p.ticket = 0u;
+    block_partial6<WBLOCK>(v, p.partials + ((uint64_t)s.part * gridDim.x + blockIdx.x) * 8);
 }
 
 // ---------------------------------------------------------------- init
@@ -1305,17 +1283,17 @@ static unsigned tma_grid() {
 
 // RAG: rows that are no whole number of 16-byte units
 template <class S, int P, int COLL, int FEAT>
-static void launch_tma(const LatParams &p, const StepParams &s, cudaStream_t st) {
+static void launch_tma(const LatParams &p, const StepParams &s, cudaStream_t st, bool pdl) {
     const unsigned ntiles = (unsigned)((p.N + Tile<S>::cells - 1) / Tile<S>::cells);
     // (ragged FP32, FP16 and BF16 lattices come here only with the regularized
     // collision and compile-time features)
     if constexpr (sizeof(S) == 8 || (COLL == 0 && FEAT != 0)) {
         if (p.ragged) {
-            k_bulk_tma<S, P, COLL, FEAT, true><<<std::min(ntiles, tma_grid<S, P, COLL, FEAT, true>()), Tma<S>::threads, tma_smem<S>(), st>>>(p, s);
+            launch_pdl(pdl, k_bulk_tma<S, P, COLL, FEAT, true>, std::min(ntiles, tma_grid<S, P, COLL, FEAT, true>()), Tma<S>::threads, tma_smem<S>(), st, p, s);
             return;
         }
     }
-    k_bulk_tma<S, P, COLL, FEAT, false><<<std::min(ntiles, tma_grid<S, P, COLL, FEAT, false>()), Tma<S>::threads, tma_smem<S>(), st>>>(p, s);
+    launch_pdl(pdl, k_bulk_tma<S, P, COLL, FEAT, false>, std::min(ntiles, tma_grid<S, P, COLL, FEAT, false>()), Tma<S>::threads, tma_smem<S>(), st, p, s);
 }
 
 uint32_t staged_tile_cells(int storage) {
@@ -1327,62 +1305,84 @@ uint32_t staged_tile_cells(int storage) {
     }
 }
 
-// one step: faces, wall cells (on the side stream `side` when they cannot
-// touch the faces' slots, overlapping the face kernel), then the bulk
+// One step: faces and wall cells, then the bulk.  Where no wall cell is near a
+// face (walls_far) the wall kernel goes first and the face kernel runs beside
+// it; in a periodic box, which has no faces, the direct bulk kernel does, from
+// the stream `side` (131x130x129 FP32: the wall kernel's 15 us beside the bulk's
+// 69 instead of before them).  The direct kernel is launched as any other, not
+// with programmatic serialization: a wait in it changes which of its products
+// the compiler fuses.  ev:
+// null, or events to record (null entries are left out); with events between
+// the kernels these run one by one.
 template <class S, int P, int COLL>
-static cudaError_t step_t(const LatParams &p, const StepParams &s, cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join,
-                          cudaEvent_t *ev) {
+static cudaError_t step_t(const LatParams &p, const StepParams &s0, cudaStream_t st, const WallsBeside &wb, cudaEvent_t *ev) {
+    const bool pdl = !(ev && ev[0]);
+    StepParams s = s0;
+    s.beside = 0;
+    const unsigned wgrid = (unsigned)((p.nrec + WBLOCK - 1) / WBLOCK);
+    auto walls = [&] { launch_pdl(pdl, k_walls<S, P, COLL>, wgrid, WBLOCK, 0, st, p, s); };
+    auto faces = [&](int beside) {
+        s.beside = beside;
+        launch_pdl(pdl, k_faces<S, P>, p.fblk[6] + blocks_for(s.nface - p.fplan[6]), BLOCK, 0, st, p, s);
+        s.beside = 0;
+    };
     if (ev && ev[0]) cudaEventRecord(ev[0], st);
     if (p.moving) {
         // re-voxelize the spinning part's swept box for this step's rotation
         // (lattice.rs:719-723): triangles -> link scratch, cells, scratch reset
-        if (p.ntri) k_tri_scatter<<<blocks_for((uint64_t)p.ntri * 32u), BLOCK, 0, st>>>(p, s);
-        k_voxelize<S, 1 - P><<<blocks_for(p.nrec), BLOCK, 0, st>>>(p, s);
-        k_qclear<<<blocks_for((uint64_t)p.nrec * 9u), BLOCK, 0, st>>>(p);
+        if (p.ntri) launch_pdl(pdl, k_tri_scatter, blocks_for((uint64_t)p.ntri * 32u), BLOCK, 0, st, p, s);
+        launch_pdl(pdl, k_voxelize<S, 1 - P>, blocks_for(p.nrec), BLOCK, 0, st, p, s);
+        launch_pdl(pdl, k_qclear, blocks_for((uint64_t)p.nrec * 9u), BLOCK, 0, st, p);
     }
-    const bool overlap = side && p.nrec && s.nface && !p.moving;
-    if (overlap) {
-        cudaEventRecord(fork, st);
-        cudaStreamWaitEvent(side, fork, 0);
-        k_walls<S, P, COLL><<<(unsigned)((p.nrec + WBLOCK - 1) / WBLOCK), WBLOCK, 0, side>>>(p, s);
-        cudaEventRecord(join, side);
-    }
-    if (s.nface) k_faces<S, P><<<p.fblk[6] + blocks_for(s.nface - p.fplan[6]), BLOCK, 0, st>>>(p, s);
+    const bool overlap = pdl && wb.far && p.nrec && s.nface && !p.moving;
+    const bool aside = pdl && wb.side && p.nrec && !p.moving;
+    if (overlap) walls();
+    if (s.nface) faces(overlap ? 1 : 0);
     if (ev && ev[1]) cudaEventRecord(ev[1], st);
-    if (overlap) cudaStreamWaitEvent(st, join, 0);
-    else if (p.nrec) k_walls<S, P, COLL><<<(unsigned)((p.nrec + WBLOCK - 1) / WBLOCK), WBLOCK, 0, st>>>(p, s);
+    if (aside) {
+        cudaEventRecord(wb.fork, st);
+        cudaStreamWaitEvent(wb.side, wb.fork, 0);
+        k_walls<S, P, COLL><<<wgrid, WBLOCK, 0, wb.side>>>(p, s);
+        cudaEventRecord(wb.join, wb.side);
+    } else if (p.nrec && !overlap) {
+        walls();
+    }
     if (ev && ev[2]) cudaEventRecord(ev[2], st);
-    // the staged kernel where it applies (lattice.cu, tma_ok), else the direct one
     if (p.tma) {
         if (!p.forcing && !p.abs_u) {
-            if (p.les_on) launch_tma<S, P, COLL, 3>(p, s, st);
-            else launch_tma<S, P, COLL, 1>(p, s, st);
+            if (p.les_on) launch_tma<S, P, COLL, 3>(p, s, st, pdl);
+            else launch_tma<S, P, COLL, 1>(p, s, st, pdl);
         } else {
-            launch_tma<S, P, COLL, 0>(p, s, st);
+            launch_tma<S, P, COLL, 0>(p, s, st, pdl);
         }
     } else {
         k_bulk<S, P, COLL><<<blocks_for(p.N), BLOCK, 0, st>>>(p, s);
     }
     if (ev && ev[3]) cudaEventRecord(ev[3], st);
+    if (aside) cudaStreamWaitEvent(st, wb.join, 0);
     return cudaGetLastError();
 }
 
 template <class S>
-static cudaError_t step_s(const LatParams &p, const StepParams &s, int parity, int coll, cudaStream_t st, cudaStream_t side, cudaEvent_t fork,
-                          cudaEvent_t join, cudaEvent_t *ev) {
-    if (parity == 0) return coll == 1 ? step_t<S, 0, 1>(p, s, st, side, fork, join, ev) : step_t<S, 0, 0>(p, s, st, side, fork, join, ev);
-    return coll == 1 ? step_t<S, 1, 1>(p, s, st, side, fork, join, ev) : step_t<S, 1, 0>(p, s, st, side, fork, join, ev);
+static cudaError_t step_s(const LatParams &p, const StepParams &s, int parity, int coll, cudaStream_t st, const WallsBeside &wb, cudaEvent_t *ev) {
+    if (parity == 0) return coll == 1 ? step_t<S, 0, 1>(p, s, st, wb, ev) : step_t<S, 0, 0>(p, s, st, wb, ev);
+    return coll == 1 ? step_t<S, 1, 1>(p, s, st, wb, ev) : step_t<S, 1, 0>(p, s, st, wb, ev);
 }
 
-cudaError_t launch_step(int storage, const LatParams &p, const StepParams &s, int parity, int coll, cudaStream_t st, cudaStream_t side,
-                        cudaEvent_t fork, cudaEvent_t join, cudaEvent_t *ev) {
+cudaError_t launch_step(int storage, const LatParams &p, const StepParams &s, int parity, int coll, cudaStream_t st, const WallsBeside &wb,
+                        cudaEvent_t *ev) {
     switch (storage) {
-        case 0: return step_s<float>(p, s, parity, coll, st, side, fork, join, ev);
-        case 1: return step_s<__half>(p, s, parity, coll, st, side, fork, join, ev);
-        case 2: return step_s<__nv_bfloat16>(p, s, parity, coll, st, side, fork, join, ev);
-        case 3: return step_s<double>(p, s, parity, coll, st, side, fork, join, ev);
+        case 0: return step_s<float>(p, s, parity, coll, st, wb, ev);
+        case 1: return step_s<__half>(p, s, parity, coll, st, wb, ev);
+        case 2: return step_s<__nv_bfloat16>(p, s, parity, coll, st, wb, ev);
+        case 3: return step_s<double>(p, s, parity, coll, st, wb, ev);
     }
     return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_force_sum(const LatParams &p, uint32_t slot0, uint32_t steps, cudaStream_t st) {
+    k_force_sum<WBLOCK><<<steps, WBLOCK, 0, st>>>(p.partials, (p.nrec + WBLOCK - 1) / WBLOCK, p.hist, slot0);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_init(int storage, const LatParams &p, cudaStream_t st) {

@@ -71,6 +71,7 @@ struct LevelParams {
     double *recd;               // FP64 engine: 6 doubles (F, T) per record
     void *wallf;                // R, 27 per record: the wall populations the step substitutes
     uint32_t nrec;
+    double *partials;           // per kept finest step and wall block: 8 doubles
     float4 *dump;
     // a spinning part on this (finest) level: every swept-box cell is a
     // record, re-voxelized each finest step from the step's rotation
@@ -93,6 +94,7 @@ struct StepArgs {
     uint32_t mw;        // moment slot this step writes (mom_child)
     uint32_t mold, mnew;  // ghost fill: the parent's moment slots at the start and end of its step
     uint32_t seed_mix;  // stochastic rounding: the step seed's term of the hash
+    uint32_t part;      // the finest step's place among the kept block partials
     float blend;        // ghost fill: time fraction between mold and mnew
     float omega[3];     // wall angular velocity, rad per finest step
     double omega_d[3];
@@ -118,10 +120,10 @@ cudaError_t launch27_sample_slices(int storage, const LevelParams &p, uint32_t s
 // block of mass27_blocks() blocks, then a u32 ticket that starts at zero
 uint32_t mass27_blocks();
 cudaError_t launch27_mass(int storage, const LevelParams &p, uint32_t src, double *scratch, double *out, cudaStream_t st);
-// FP64 sum of the records' force and moment into out[0..5] (deterministic
-// order: per-block partials, the last block sums them)
-cudaError_t launch27_reduce(const LevelParams &p, int fp64, double *partials, uint32_t *ticket, double *out, cudaStream_t st);
-uint32_t reduce27_blocks(uint32_t nrec);
+// FP64 force and moment of the finest steps whose partials are kept, into the
+// history slots slot0, slot0 + 1, ...
+cudaError_t launch27_force_sum(const LevelParams &p, double *hist, uint32_t slot0, uint32_t steps, cudaStream_t st);
+uint32_t walls27_blocks(uint32_t nrec);
 // re-voxelize the spinning part's swept box for the rotation in `a` (finest level)
 cudaError_t launch27_revoxel(int storage, const LevelParams &p, const StepArgs &a, cudaStream_t st);
 

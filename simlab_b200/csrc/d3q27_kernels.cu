@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "d3q27.h"
+#include "pdl.cuh"
 #include "spin_math.cuh"
 #include "reduce.cuh"
 
@@ -459,14 +460,13 @@ template <class S> struct WallOcc { static constexpr int value = 3; };
 template <> struct WallOcc<double> { static constexpr int value = 1; };
 
 template <class S>
-__global__ void __launch_bounds__(BLK, WallOcc<S>::value) k27_walls(const __grid_constant__ LevelParams p, const StepArgs a) {
+__device__ __forceinline__ bool wall_record(const LevelParams &p, const StepArgs &a, uint32_t r, double *v) {
     using R = typename Pop<S>::real;
-    const uint32_t r = blockIdx.x * BLK + threadIdx.x;
-    if (r >= p.nrec) return;
+    if (r >= p.nrec) return true;
     const uint32_t n = p.recs[r * RS + R_CELL];
     const uint32_t fg = p.flags[n];
     // only the cells the step updates, each through its own record
-    if ((fg & 7u) != 0 || (fg >> 3) != r + 1) return;
+    if ((fg & 7u) != 0 || (fg >> 3) != r + 1) return false;
     uint32_t x, y, z;
     coords(p, n, x, y, z);
     const Consts27<R> &k = K<R>(p);
@@ -550,11 +550,30 @@ __global__ void __launch_bounds__(BLK, WallOcc<S>::value) k27_walls(const __grid
     if (p.recd) {
         for (int c = 0; c < 3; c++) { p.recd[r * 6 + c] = (double)Fv[c]; p.recd[r * 6 + 3 + c] = (double)Tv[c]; }
     }
+    for (int c = 0; c < 3; c++) { v[c] = (double)Fv[c]; v[3 + c] = (double)Tv[c]; }
+    return true;
+}
+
+template <class S>
+__global__ void __launch_bounds__(BLK, WallOcc<S>::value) k27_walls(const __grid_constant__ LevelParams p, const __grid_constant__ StepArgs a) {
+    lbm::pdl_release();
+    lbm::pdl_wait();
+    const uint32_t r = blockIdx.x * BLK + threadIdx.x;
+    // every record's force and moment enters the step's sum (mshader.rs:519-562
+    // sums them in f32), those the step does not update as they stand
+    double v[6] = {0, 0, 0, 0, 0, 0};
+    if (!wall_record<S>(p, a, r, v)) {
+#pragma unroll
+        for (int j = 0; j < 6; j++) v[j] = p.recd ? p.recd[(uint64_t)r * 6 + j] : (double)__uint_as_float(p.recs[(uint64_t)r * RS + R_FT + j]);
+    }
+    lbm::block_partial6<BLK>(v, p.partials + ((uint64_t)a.part * gridDim.x + blockIdx.x) * 8);
 }
 
 template <class S, bool FORCE, bool WRAP, bool SPONGE>
 __global__ void __launch_bounds__(BLK, StepOcc<S, WRAP, SPONGE>::value) k27_step(const __grid_constant__ LevelParams p, const StepArgs a) {
     using R = typename Pop<S>::real;
+    lbm::pdl_release();
+    lbm::pdl_wait();
     const uint32_t n = blockIdx.x * BLK + threadIdx.x;
     if (n >= p.N) return;
     const uint32_t fg = p.flags[n];
@@ -586,6 +605,8 @@ __global__ void __launch_bounds__(BLK, StepOcc<S, WRAP, SPONGE>::value) k27_step
 template <class S>
 __global__ void __launch_bounds__(BLK) k27_face(const __grid_constant__ LevelParams p, const StepArgs a) {
     using R = typename Pop<S>::real;
+    lbm::pdl_release();
+    lbm::pdl_wait();
     const uint32_t kk = blockIdx.x * BLK + threadIdx.x;
     if (kk >= p.nface) return;
     const Consts27<R> &k = K<R>(p);
@@ -630,6 +651,8 @@ __global__ void __launch_bounds__(BLK) k27_face(const __grid_constant__ LevelPar
 template <class S>
 __global__ void __launch_bounds__(BLK) k27_ghost(const __grid_constant__ LevelParams p, const StepArgs a) {
     using R = typename Pop<S>::real;
+    lbm::pdl_release();
+    lbm::pdl_wait();
     const uint32_t kk = blockIdx.x * BLK + threadIdx.x;
     if (kk >= p.nghost) return;
     const uint32_t n = p.ghosts[kk];
@@ -674,6 +697,8 @@ __global__ void __launch_bounds__(BLK) k27_ghost(const __grid_constant__ LevelPa
 template <class S>
 __global__ void __launch_bounds__(BLK) k27_restrict(const __grid_constant__ LevelParams p, const StepArgs a) {
     using R = typename Pop<S>::real;
+    lbm::pdl_release();
+    lbm::pdl_wait();
     const uint32_t kk = blockIdx.x * BLK + threadIdx.x;
     if (kk >= p.nrestrict) return;
     const uint32_t n = p.restricted[kk];
@@ -795,12 +820,6 @@ __global__ void __launch_bounds__(BLK) k27_sample_slices(const __grid_constant__
     }
 }
 
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // FP64 mass and non-finite count of the plain fluid cells of a level:
 // grid-stride over the cells, then the deterministic grid sum of reduce.cuh
 // (one atomic per block; the same result on every run).  out[0] = mass,
@@ -844,6 +863,8 @@ __device__ __forceinline__ bool in_box(const LevelParams &p, int lx, int ly, int
 
 __global__ void __launch_bounds__(BLK) k27_tri_scatter(const __grid_constant__ LevelParams p, const StepArgs a) {
     using namespace lbm::rv;
+    lbm::pdl_release();
+    lbm::pdl_wait();
     // one warp per triangle, its lanes over the lattice points near it
     const uint32_t t = (blockIdx.x * BLK + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
     if (t >= p.ntri) return;
@@ -891,6 +912,8 @@ __global__ void __launch_bounds__(BLK) k27_tri_scatter(const __grid_constant__ L
 }
 
 __global__ void __launch_bounds__(BLK) k27_qclear(const __grid_constant__ LevelParams p) {
+    lbm::pdl_release();
+    lbm::pdl_wait();
     const uint64_t k = (uint64_t)blockIdx.x * BLK + threadIdx.x;
     if (k >= (uint64_t)p.nrec * 13u) return;
     p.qscr[3 * k] = 0x7f7fffffu;
@@ -902,6 +925,8 @@ template <class S>
 __global__ void __launch_bounds__(BLK) k27_voxelize(const __grid_constant__ LevelParams p, const StepArgs a) {
     using namespace lbm::rv;
     using R = typename Pop<S>::real;
+    lbm::pdl_release();
+    lbm::pdl_wait();
     const uint32_t k = blockIdx.x * BLK + threadIdx.x;
     if (k >= p.nrec) return;
     const int lx = (int)(k % p.box_n[0]), ly = (int)((k / p.box_n[0]) % p.box_n[1]), lz = (int)(k / (p.box_n[0] * p.box_n[1]));
@@ -1005,53 +1030,6 @@ __global__ void __launch_bounds__(BLK) k27_voxelize(const __grid_constant__ Leve
         for (int c = 0; c < 3; c++) { p.recd[k * 6 + c] = (double)F[c]; p.recd[k * 6 + 3 + c] = (double)T[c]; }
 }
 
-// FP64 sum of the records' force and moment: per-block partials in fixed
-// order, the last block to finish sums the partials (mshader.rs:519-562 does
-// the same sum in f32)
-constexpr uint32_t RED_BLK = 256;
-template <bool FP64>
-__global__ void __launch_bounds__(RED_BLK) k27_reduce(const __grid_constant__ LevelParams p, double *partials, uint32_t *ticket, double *out) {
-    const uint32_t r = blockIdx.x * RED_BLK + threadIdx.x;
-    double v[6] = {0, 0, 0, 0, 0, 0};
-    if (r < p.nrec) {
-#pragma unroll
-        for (int j = 0; j < 6; j++) v[j] = FP64 ? p.recd[(uint64_t)r * 6 + j] : (double)__uint_as_float(p.recs[(uint64_t)r * RS + R_FT + j]);
-    }
-    __shared__ double sh[RED_BLK / 32][6];
-    __shared__ bool last;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int j = 0; j < 6; j++) v[j] = warp_sum(v[j]);
-    if (lane == 0)
-        for (int j = 0; j < 6; j++) sh[warp][j] = v[j];
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        double t = 0;
-        for (int w = 0; w < (int)(RED_BLK / 32); w++) t += sh[w][threadIdx.x];
-        partials[blockIdx.x * 8 + threadIdx.x] = t;
-        __threadfence();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (uint32_t b = threadIdx.x; b < gridDim.x; b += RED_BLK)
-        for (int j = 0; j < 6; j++) acc[j] += __ldcg(&partials[b * 8 + j]);
-    for (int j = 0; j < 6; j++) acc[j] = warp_sum(acc[j]);
-    __syncthreads();
-    if (lane == 0)
-        for (int j = 0; j < 6; j++) sh[warp][j] = acc[j];
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        double t = 0;
-        for (int w = 0; w < (int)(RED_BLK / 32); w++) t += sh[w][threadIdx.x];
-        out[threadIdx.x] = t;
-    }
-    if (threadIdx.x == 0) *ticket = 0u;
-}
-
 // ------------------------------------------------------------ launchers
 static inline unsigned blocks_for(uint64_t n) { return (unsigned)((n + BLK - 1) / BLK); }
 
@@ -1078,7 +1056,7 @@ cudaError_t launch27_face(int storage, const LevelParams &p, const StepArgs &a, 
     if (!p.nface) return cudaSuccess;
     return dispatch(storage, [&](auto *t) {
         using S = std::remove_pointer_t<decltype(t)>;
-        k27_face<S><<<blocks_for(p.nface), BLK, 0, st>>>(p, a);
+        lbm::launch_pdl(true, k27_face<S>, blocks_for(p.nface), BLK, 0, st, p, a);
         return cudaGetLastError();
     });
 }
@@ -1089,22 +1067,22 @@ cudaError_t launch27_step(int storage, const LevelParams &p, const StepArgs &a, 
         const bool wrap = p.per[0] || p.per[1] || p.per[2];
         const unsigned g = blocks_for(p.N);
         const bool sp = p.n_sponge != 0;
-        if (p.nrec) k27_walls<S><<<blocks_for(p.nrec), BLK, 0, st>>>(p, a);
+        if (p.nrec) lbm::launch_pdl(true, k27_walls<S>, blocks_for(p.nrec), BLK, 0, st, p, a);
         if (p.forcing) {
             if (wrap) {
-                if (sp) k27_step<S, true, true, true><<<g, BLK, 0, st>>>(p, a);
-                else k27_step<S, true, true, false><<<g, BLK, 0, st>>>(p, a);
+                if (sp) lbm::launch_pdl(true, k27_step<S, true, true, true>, g, BLK, 0, st, p, a);
+                else lbm::launch_pdl(true, k27_step<S, true, true, false>, g, BLK, 0, st, p, a);
             } else {
-                if (sp) k27_step<S, true, false, true><<<g, BLK, 0, st>>>(p, a);
-                else k27_step<S, true, false, false><<<g, BLK, 0, st>>>(p, a);
+                if (sp) lbm::launch_pdl(true, k27_step<S, true, false, true>, g, BLK, 0, st, p, a);
+                else lbm::launch_pdl(true, k27_step<S, true, false, false>, g, BLK, 0, st, p, a);
             }
         } else {
             if (wrap) {
-                if (sp) k27_step<S, false, true, true><<<g, BLK, 0, st>>>(p, a);
-                else k27_step<S, false, true, false><<<g, BLK, 0, st>>>(p, a);
+                if (sp) lbm::launch_pdl(true, k27_step<S, false, true, true>, g, BLK, 0, st, p, a);
+                else lbm::launch_pdl(true, k27_step<S, false, true, false>, g, BLK, 0, st, p, a);
             } else {
-                if (sp) k27_step<S, false, false, true><<<g, BLK, 0, st>>>(p, a);
-                else k27_step<S, false, false, false><<<g, BLK, 0, st>>>(p, a);
+                if (sp) lbm::launch_pdl(true, k27_step<S, false, false, true>, g, BLK, 0, st, p, a);
+                else lbm::launch_pdl(true, k27_step<S, false, false, false>, g, BLK, 0, st, p, a);
             }
         }
         return cudaGetLastError();
@@ -1115,7 +1093,7 @@ cudaError_t launch27_ghost(int storage, const LevelParams &p, const StepArgs &a,
     if (!p.nghost) return cudaSuccess;
     return dispatch(storage, [&](auto *t) {
         using S = std::remove_pointer_t<decltype(t)>;
-        k27_ghost<S><<<blocks_for(p.nghost), BLK, 0, st>>>(p, a);
+        lbm::launch_pdl(true, k27_ghost<S>, blocks_for(p.nghost), BLK, 0, st, p, a);
         return cudaGetLastError();
     });
 }
@@ -1124,7 +1102,7 @@ cudaError_t launch27_restrict(int storage, const LevelParams &p, const StepArgs 
     if (!p.nrestrict) return cudaSuccess;
     return dispatch(storage, [&](auto *t) {
         using S = std::remove_pointer_t<decltype(t)>;
-        k27_restrict<S><<<blocks_for(p.nrestrict), BLK, 0, st>>>(p, a);
+        lbm::launch_pdl(true, k27_restrict<S>, blocks_for(p.nrestrict), BLK, 0, st, p, a);
         return cudaGetLastError();
     });
 }
@@ -1177,26 +1155,23 @@ cudaError_t launch27_mass(int storage, const LevelParams &p, uint32_t src, doubl
     });
 }
 
-uint32_t reduce27_blocks(uint32_t nrec) { return (nrec + RED_BLK - 1) / RED_BLK; }
+uint32_t walls27_blocks(uint32_t nrec) { return (nrec + BLK - 1) / BLK; }
 
 cudaError_t launch27_revoxel(int storage, const LevelParams &p, const StepArgs &a, cudaStream_t st) {
     if (!p.moving) return cudaSuccess;
-    if (p.ntri) k27_tri_scatter<<<blocks_for((uint64_t)p.ntri * 32u), BLK, 0, st>>>(p, a);
+    if (p.ntri) lbm::launch_pdl(true, k27_tri_scatter, blocks_for((uint64_t)p.ntri * 32u), BLK, 0, st, p, a);
     cudaError_t e = dispatch(storage, [&](auto *t) {
         using S = std::remove_pointer_t<decltype(t)>;
-        k27_voxelize<S><<<blocks_for(p.nrec), BLK, 0, st>>>(p, a);
+        lbm::launch_pdl(true, k27_voxelize<S>, blocks_for(p.nrec), BLK, 0, st, p, a);
         return cudaGetLastError();
     });
     if (e != cudaSuccess) return e;
-    k27_qclear<<<blocks_for((uint64_t)p.nrec * 13u), BLK, 0, st>>>(p);
+    lbm::launch_pdl(true, k27_qclear, blocks_for((uint64_t)p.nrec * 13u), BLK, 0, st, p);
     return cudaGetLastError();
 }
 
-cudaError_t launch27_reduce(const LevelParams &p, int fp64, double *partials, uint32_t *ticket, double *out, cudaStream_t st) {
-    if (p.nrec == 0) return cudaMemsetAsync(out, 0, 6 * sizeof(double), st);
-    const uint32_t nb = reduce27_blocks(p.nrec);
-    if (fp64) k27_reduce<true><<<nb, RED_BLK, 0, st>>>(p, partials, ticket, out);
-    else k27_reduce<false><<<nb, RED_BLK, 0, st>>>(p, partials, ticket, out);
+cudaError_t launch27_force_sum(const LevelParams &p, double *hist, uint32_t slot0, uint32_t steps, cudaStream_t st) {
+    lbm::k_force_sum<BLK><<<steps, BLK, 0, st>>>(p.partials, walls27_blocks(p.nrec), hist, slot0);
     return cudaGetLastError();
 }
 

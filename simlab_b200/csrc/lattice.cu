@@ -20,11 +20,8 @@
 #include "../../include/simlab_lbm.h"
 #include "host_wait.hpp"
 #include "lbm_kernels.h"
+#include "reduce.cuh"
 #include "voxel.hpp"
-
-#ifndef LBM_SIDE_PRIORITY
-#define LBM_SIDE_PRIORITY 1  // wall-cell stream at the device's greatest priority
-#endif
 
 namespace {
 
@@ -74,8 +71,8 @@ struct lbm_lattice {
     lbm_setup setup{};
     lbm::LatParams lp{};
     cudaStream_t stream = nullptr;
-    cudaStream_t side = nullptr;  // wall-cell kernel, when it cannot touch the faces' slots
-    cudaEvent_t fork = nullptr, join = nullptr;
+    lbm::WallsBeside walls_beside;
+    uint32_t ring = 1;       // steps whose wall-kernel partials are kept before they are summed
     int device = 0;
     std::vector<void *> allocs;
     uint64_t steps_done = 0;
@@ -115,8 +112,9 @@ struct lbm_lattice {
     ~lbm_lattice() {
         // bounded waits: if the device never finishes, the buffers it may
         // still use are left allocated rather than freed under it
+        lbm::WallsBeside &wb = walls_beside;
         if ((stream && lbm::stream_wait(stream, timeout_s) == cudaErrorTimeout) ||
-            (side && lbm::stream_wait(side, timeout_s) == cudaErrorTimeout)) {
+            (wb.side && lbm::stream_wait(wb.side, timeout_s) == cudaErrorTimeout)) {
             lbm_host::set_global_error("lattice destroyed while its device work had not finished: buffers left allocated");
             return;
         }
@@ -125,9 +123,9 @@ struct lbm_lattice {
         if (err_host) cudaFreeHost(err_host);
         if (ev) cudaEventDestroy(ev);
         for (cudaEvent_t e : prof_ev) cudaEventDestroy(e);
-        if (fork) cudaEventDestroy(fork);
-        if (join) cudaEventDestroy(join);
-        if (side) cudaStreamDestroy(side);
+        if (wb.fork) cudaEventDestroy(wb.fork);
+        if (wb.join) cudaEventDestroy(wb.join);
+        if (wb.side) cudaStreamDestroy(wb.side);
         if (stream) cudaStreamDestroy(stream);
     }
     void wait() {
@@ -206,7 +204,7 @@ lbm::StepParams step_params(const lbm_lattice *h, const lbm_step_in &s, uint32_t
     sp.seed_mix = sp.seed * 0x85EBCA77u + 0x632BE5ABu;
     sp.next_seed_mix = ((uint32_t)(step_index + 1) * lbm::STEP_SEED_MUL) * 0x85EBCA77u + 0x632BE5ABu;
     sp.nface = h->fused_valid ? h->nface_rest : h->nface;
-    sp.slot = slot;
+    sp.part = slot % h->ring;
     for (int a = 0; a < 3; a++) {
         sp.omega[a] = (float)s.omega[a];
         sp.omega_d[a] = s.omega[a];
@@ -536,8 +534,8 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
     p.faces = (uint32_t *)h->dalloc(faces.size() * 4);
     p.face_info = (uint32_t *)h->dalloc(finfo.size() * 4);
     const uint64_t nwb = (nrec + lbm::WBLOCK - 1) / lbm::WBLOCK;  // blocks of the wall-cell kernel
-    p.partials = (double *)h->dalloc(std::max<uint64_t>(nwb, 1) * 8 * sizeof(double));
-    p.ticket = (uint32_t *)h->dalloc(16);
+    h->ring = lbm::force_ring(std::max<uint64_t>(nwb, 1), KMAX);
+    p.partials = (double *)h->dalloc((uint64_t)h->ring * std::max<uint64_t>(nwb, 1) * 8 * sizeof(double));
     p.hist = (double *)h->dalloc(KMAX * 8 * sizeof(double));
     p.dump = st.debug_dump ? (float4 *)h->dalloc(N * 16) : nullptr;
     h->vacc = (double *)h->dalloc(std::max<uint64_t>(h->nvert, 1) * 2 * sizeof(double));
@@ -649,16 +647,12 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
     ck(cudaMemcpyAsync(h->slicedef, sd.data(), sd.size() * 4, cudaMemcpyHostToDevice, s), "upload slices");
     ck(cudaMemcpyAsync((void *)p.sp_tab, tabf.data(), tabf.size() * 4, cudaMemcpyHostToDevice, s), "upload sponge");
     ck(cudaMemcpyAsync((void *)p.sp_tabd, tabd.data(), tabd.size() * 8, cudaMemcpyHostToDevice, s), "upload sponge");
-    if (walls_far) {
-        // the wall-cell kernel is the longer of the two that run before the
-        // bulk: its blocks go first on the SMs
-        int prio_lo = 0, prio_hi = 0;
-        ck(cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi), "cudaDeviceGetStreamPriorityRange");
-        ck(cudaStreamCreateWithPriority(&h->side, cudaStreamNonBlocking, LBM_SIDE_PRIORITY ? prio_hi : prio_lo), "cudaStreamCreate");
-        ck(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming), "cudaEventCreate");
-        ck(cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming), "cudaEventCreate");
+    h->walls_beside.far = walls_far;
+    if (nrec > 0 && faces.empty() && !spin) {
+        ck(cudaStreamCreateWithFlags(&h->walls_beside.side, cudaStreamNonBlocking), "cudaStreamCreate");
+        ck(cudaEventCreateWithFlags(&h->walls_beside.fork, cudaEventDisableTiming), "cudaEventCreate");
+        ck(cudaEventCreateWithFlags(&h->walls_beside.join, cudaEventDisableTiming), "cudaEventCreate");
     }
-    ck(cudaMemsetAsync(p.ticket, 0, 16, s), "memset");
     ck(cudaMemsetAsync(p.hist, 0, KMAX * 8 * sizeof(double), s), "memset");
     ck(cudaMemsetAsync(h->vacc, 0, std::max<uint64_t>(h->nvert, 1) * 2 * sizeof(double), s), "memset");
     ck(cudaMemsetAsync(h->sacc, 0, std::max<uint64_t>(h->npix, 1) * 5 * sizeof(double), s), "memset");
@@ -698,7 +692,7 @@ void run_impl(lbm_lattice *h, const lbm_step_in *steps, uint64_t n, double *forc
                 h->prof_launches += (sp.nface ? 1u : 0u) + (p.nrec ? 1u : 0u) + 1u + (p.moving ? 2u + (p.ntri ? 1u : 0u) : 0u);
                 if (si.sample) h->prof_launches += (h->nvert ? 1u : 0u) + (h->npix ? 1u : 0u);
             }
-            ck(lbm::launch_step(h->setup.storage, p, sp, (int)(idx % 2), h->setup.collision, h->stream, h->side, h->fork, h->join, evs),
+            ck(lbm::launch_step(h->setup.storage, p, sp, (int)(idx % 2), h->setup.collision, h->stream, h->walls_beside, evs),
                "step kernels");
             if (si.sample && (h->nvert || h->npix))
                 ck(lbm::launch_sample(h->setup.storage, p, sp, (int)(idx % 2), h->verts, h->nvert, h->voff, h->vacc, h->slicedef,
@@ -706,6 +700,8 @@ void run_impl(lbm_lattice *h, const lbm_step_in *steps, uint64_t n, double *forc
                    "sample kernels");
             h->steps_done++;
             h->fused_valid = h->xfuse;
+            if (p.nrec && ((k + 1) % h->ring == 0 || k + 1 == len))
+                ck(lbm::launch_force_sum(p, k - k % h->ring, k % h->ring + 1, h->stream), "force sum");
         }
         if (readback) {
             ck(cudaMemcpyAsync(h->hist_host, p.hist, len * 8 * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "history readback");

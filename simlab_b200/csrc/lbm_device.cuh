@@ -120,8 +120,7 @@ struct LatParams {
     double *recd;              // FP64 engine: nrec * RD doubles (else null)
     const uint32_t *faces;     // face cells
     const uint32_t *face_info; // kind (0 velocity, 1 open, 2 free slip) | mirror axes << 2 | store mask << 8
-    double *partials;          // per wall block: 8 doubles
-    uint32_t *ticket;          // last-block counter of the force reduction
+    double *partials;          // per kept step and wall block: 8 doubles
     double *hist;              // per step slot: 8 doubles (F, T)
     float4 *dump;              // macros() output
     uint32_t *err;             // error bits (ERR_*)
@@ -172,7 +171,8 @@ struct StepParams {
     uint32_t seed_mix;  // seed * 0x85EBCA77 + 0x632BE5AB, the seed's term of sr_hash
     uint32_t next_seed_mix;  // the same for the next step
     uint32_t nface;          // face cells the face kernel handles this step
-    uint32_t slot;   // history slot of this step
+    uint32_t part;   // the step's place among the kept block partials
+    int beside;      // this kernel runs beside the wall kernel, not after it
     float omega[3];  // angular velocity, rad per step
     double omega_d[3];
     float rot[9];    // body axes in lattice coordinates, row-major (columns = axes)

@@ -7,11 +7,21 @@
 namespace lbm {
 
 // storage: 0 FP32, 1 FP16, 2 BF16, 3 FP64 (lbm_storage); coll: 0 regularized, 1 BGK
-// side: null, or a second stream on which the wall-cell kernel overlaps the
-// face kernel (fork/join: two events); ev: null, or 4 events recorded before
-// the step, after faces, after walls, after bulk
-cudaError_t launch_step(int storage, const LatParams &p, const StepParams &s, int parity, int coll, cudaStream_t st, cudaStream_t side,
-                        cudaEvent_t fork, cudaEvent_t join, cudaEvent_t *ev = nullptr);
+// What the wall kernel may run beside: the face kernel (far: no wall cell is
+// near a face), or the direct bulk kernel of a lattice without faces, from a
+// second stream (side, with the two events that fork it off and join it).
+struct WallsBeside {
+    bool far = false;
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+};
+// ev: null, or 4 events recorded before the step, after faces,
+// after walls, after bulk
+cudaError_t launch_step(int storage, const LatParams &p, const StepParams &s, int parity, int coll, cudaStream_t st, const WallsBeside &wb,
+                        cudaEvent_t *ev = nullptr);
+// force and moment of the steps whose partials are kept, into the history
+// slots slot0, slot0 + 1, ...
+cudaError_t launch_force_sum(const LatParams &p, uint32_t slot0, uint32_t steps, cudaStream_t st);
 // cells of one tile of the staged bulk kernel: tiles start at its multiples
 uint32_t staged_tile_cells(int storage);
 cudaError_t launch_init(int storage, const LatParams &p, cudaStream_t st);

@@ -23,6 +23,7 @@
 #include "../../include/simlab_lbm.h"
 #include "d3q27.h"
 #include "host_wait.hpp"
+#include "reduce.cuh"
 
 namespace lbm_host {
 void set_global_error(const std::string &msg);
@@ -84,7 +85,7 @@ struct lbm_multi {
     double *recd = nullptr;
     void *wallf = nullptr;  // 27 reals per record, written by the wall kernel each finest step
     double *partials = nullptr;
-    uint32_t *ticket = nullptr;
+    uint32_t ring = 1;            // finest steps whose wall-kernel partials are kept before they are summed
     double *hist = nullptr;       // HIST_CAP x 8 doubles
     double *hist_host = nullptr;  // pinned
     double *mass_d = nullptr;   // mass, non-finite count, then the grid sum's block partials and ticket
@@ -137,6 +138,10 @@ struct lbm_multi {
     }
     static uint32_t mix(uint32_t seed) { return seed * 0x85EBCA77u + 0x632BE5ABu; }
 
+    void sum_forces(size_t first, size_t count) {
+        ck(lbm27::launch27_force_sum(lv.back().p, hist, (uint32_t)first, (uint32_t)count, stream), "force sum");
+    }
+
     // mlattice.rs:786-842: one step of level l and, nested in it, two steps
     // of each finer level with their ghost fills, then the restriction
     void schedule(size_t l, const lbm_step_in *fine, size_t &fine_i) {
@@ -147,6 +152,7 @@ struct lbm_multi {
         lbm27::StepArgs a{};
         a.src = lsrc;
         a.mw = lmw;
+        a.part = (uint32_t)(fine_i % ring);
         a.seed_mix = mix(seed_of(hslot, lsrc, lmw));
         for (int k = 0; k < 9; k++) a.rot[k] = a.rot_prev[k] = (k % 4 == 0) ? 1.0f : 0.0f;
         if (l == finest && fine) {
@@ -164,7 +170,6 @@ struct lbm_multi {
         L.mslot = lmw;
         L.steps++;
         if (l == finest) {
-            ck(lbm27::launch27_reduce(L.p, storage == LBM_STORAGE_FP64, partials, ticket, hist + (fine_i % HIST_CAP) * 8, stream), "reduce kernel");
             if (fine && fine[fine_i].sample) {
                 // mlattice.rs:812-824: vertices with this step's rotation on the
                 // finest level's new state, then the slices of every level
@@ -175,6 +180,7 @@ struct lbm_multi {
                     ck(lbm27::launch27_sample_slices(storage, lv[q].p, lv[q].src, pix[q], npix_l[q], sacc, stream), "slice probes");
             }
             fine_i++;
+            if (nrec && fine_i % ring == 0) sum_forces(fine_i - ring, ring);
         }
         if (l + 1 < nl) {
             const uint32_t mold = 1u - lmw;
@@ -205,8 +211,10 @@ struct lbm_multi {
         while (done < n) {
             const size_t nc = std::min<uint64_t>((n - done) / ss, max_coarse);
             size_t fine_i = 0;
-            for (size_t k = 0; k < nc; k++) schedule(0, fine ? fine + done : nullptr, fine_i);
             const size_t nf = nc * ss;
+            if (!nrec) ck(cudaMemsetAsync(hist, 0, nf * 8 * sizeof(double), stream), "memset");
+            for (size_t k = 0; k < nc; k++) schedule(0, fine ? fine + done : nullptr, fine_i);
+            if (nrec && nf % ring != 0) sum_forces(nf - nf % ring, nf % ring);
             if (forces) {
                 ck(cudaMemcpyAsync(hist_host, hist, nf * 8 * sizeof(double), cudaMemcpyDeviceToHost, stream), "history readback");
                 wait();
@@ -539,9 +547,9 @@ void create_multi(const lbm_multi_setup *setup, const lbm_geometry *geom, const 
         ck(cudaMemsetAsync(h->recd, 0, std::max<uint64_t>(nrec, 1) * 6 * 8, h->stream), "records init");
     }
     h->wallf = h->dalloc(std::max<uint64_t>(nrec, 1) * 27 * rsz);
-    h->partials = (double *)h->dalloc((size_t)std::max<uint32_t>(lbm27::reduce27_blocks(h->nrec), 1) * 8 * 8);
-    h->ticket = (uint32_t *)h->dalloc(16);
-    ck(cudaMemsetAsync(h->ticket, 0, 16, h->stream), "ticket init");
+    const uint32_t nwb = std::max<uint32_t>(lbm27::walls27_blocks(h->nrec), 1);
+    h->ring = lbm::force_ring(nwb, (uint32_t)HIST_CAP);
+    h->partials = (double *)h->dalloc((size_t)h->ring * nwb * 8 * 8);
     h->hist = (double *)h->dalloc(HIST_CAP * 8 * 8);
     ck(cudaMemsetAsync(h->hist, 0, HIST_CAP * 8 * 8, h->stream), "history init");
     h->verts = (float *)h->dalloc(std::max<size_t>(vbuf.size(), 8) * 4);
@@ -586,8 +594,8 @@ void create_multi(const lbm_multi_setup *setup, const lbm_geometry *geom, const 
     for (size_t l = 0; l < nl; l++) {
         lbm27::LevelParams &p = h->lv[l].p;
         p.dump = h->dump;
-        if (l == finest) { p.recs = h->recs; p.recd = h->recd; p.wallf = h->wallf; p.nrec = h->nrec; }
-        else { p.recs = nullptr; p.recd = nullptr; p.wallf = nullptr; p.nrec = 0; }
+        if (l == finest) { p.recs = h->recs; p.recd = h->recd; p.wallf = h->wallf; p.nrec = h->nrec; p.partials = h->partials; }
+        else { p.recs = nullptr; p.recd = nullptr; p.wallf = nullptr; p.nrec = 0; p.partials = nullptr; }
         ck(lbm27::launch27_init(s.storage, p, h->stream), "init kernel");
     }
     h->wait();

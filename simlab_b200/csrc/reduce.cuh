@@ -58,4 +58,53 @@ __device__ __forceinline__ void grid_sum2(double a, double b, double *scratch, d
     }
 }
 
+// The force and moment of each step of a batch from the wall kernel's block
+// partials (6 doubles, 8 apart; nblk blocks per step, the steps one after
+// another): block k sums step slot0 + k in block order into hist.  Left to one
+// launch per batch: summed by the wall kernel's last block, every step paid
+// for the fence, the counter and the second pass (3-5 us) before the bulk.
+template <int NT>
+__global__ void __launch_bounds__(NT) k_force_sum(const double *__restrict__ partials, uint32_t nblk, double *__restrict__ hist, uint32_t slot0) {
+    __shared__ double sh[NT / 32][6];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double *part = partials + (uint64_t)blockIdx.x * nblk * 8;
+    double acc[6] = {0, 0, 0, 0, 0, 0};
+    for (uint32_t b = threadIdx.x; b < nblk; b += NT)
+        for (int j = 0; j < 6; j++) acc[j] += part[(uint64_t)b * 8 + j];
+#pragma unroll
+    for (int j = 0; j < 6; j++) acc[j] = warp_sum_d(acc[j]);
+    if (lane == 0)
+        for (int j = 0; j < 6; j++) sh[warp][j] = acc[j];
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        double t = 0;
+        for (int w = 0; w < NT / 32; w++) t += sh[w][threadIdx.x];
+        hist[(uint64_t)(slot0 + blockIdx.x) * 8 + threadIdx.x] = t;
+    }
+}
+
+// A block's 6 sums into its partial (warp shuffles, then the warps in order).
+template <int NT>
+__device__ __forceinline__ void block_partial6(double *v, double *out) {
+    __shared__ double sh[NT / 32][6];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int j = 0; j < 6; j++) v[j] = warp_sum_d(v[j]);
+    if (lane == 0)
+        for (int j = 0; j < 6; j++) sh[warp][j] = v[j];
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        double t = 0;
+        for (int w = 0; w < NT / 32; w++) t += sh[w][threadIdx.x];
+        out[threadIdx.x] = t;
+    }
+}
+
+// steps whose partials are kept before they are summed: as many of `most` as
+// 16 MB hold
+inline uint32_t force_ring(uint64_t nblk, uint32_t most) {
+    const uint64_t n = (16ull << 20) / (nblk * 64);
+    return n < 1 ? 1u : (n > most ? most : (uint32_t)n);
+}
+
 }  // namespace lbm

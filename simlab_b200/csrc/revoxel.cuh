@@ -17,6 +17,7 @@
 #pragma once
 
 #include "lbm_device.cuh"
+#include "pdl.cuh"
 #include "spin_math.cuh"
 
 namespace lbm {
@@ -34,6 +35,8 @@ __device__ __forceinline__ bool solid_at(const LatParams &p, const StepParams &s
 // shader.rs:902-940: one thread per triangle
 __global__ void __launch_bounds__(BLOCK) k_tri_scatter(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
     using namespace rv;
+    pdl_release();
+    pdl_wait();
     // one warp per triangle, its lanes over the lattice points near it
     const uint32_t t = (blockIdx.x * BLOCK + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
     if (t >= p.ntri) return;
@@ -80,6 +83,8 @@ __global__ void __launch_bounds__(BLOCK) k_tri_scatter(const __grid_constant__ L
 
 // shader.rs:942-948
 __global__ void __launch_bounds__(BLOCK) k_qclear(const __grid_constant__ LatParams p) {
+    pdl_release();
+    pdl_wait();
     const uint64_t k = (uint64_t)blockIdx.x * BLOCK + threadIdx.x;
     if (k >= (uint64_t)p.nrec * 9u) return;
     p.qscr[3 * k] = 0x7f7fffffu;
@@ -94,6 +99,8 @@ template <class S, int Q>
 __global__ void __launch_bounds__(BLOCK) k_voxelize(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
     using namespace rv;
     using R = typename Pop<S>::real;
+    pdl_release();
+    pdl_wait();
     const uint32_t k = blockIdx.x * BLOCK + threadIdx.x;
     if (k >= p.nrec) return;
     const uint32_t lx = k % p.box_n[0], ly = (k / p.box_n[0]) % p.box_n[1], lz = k / (p.box_n[0] * p.box_n[1]);
