@@ -554,7 +554,9 @@ __global__ void __launch_bounds__(BLOCK) k_faces(const __grid_constant__ LatPara
 // 20 warps with three buffers of 1280 / 640 cells 46.3 / 34.6 k; one block of
 // 20 warps with two buffers of 2560 / 1280 cells 56.4 / 38.9 k; the same with
 // 2, 3, 4, 5 producer warps 59.8, 60.3, 60.5, 58.7 k FP16 (FP32 38.2 k with 2 or
-// 3).  The copy engine takes a few hundred cycles per bulk copy (one per plane
+// 3).  With two cells per thread (bulk_pairs), us per FP16 step: 20 warps and
+// 2560 cells 493, 16 and 2048 537, 14 and 2688 525, 12 and 2304 557, 10 and
+// 2560 572, so the shape stays.  The copy engine takes a few hundred cycles per bulk copy (one per plane
 // and tile, each way) and the copies one warp issues go one after another, so
 // fewer, larger copies and several issuing warps shorten a buffer's
 // turnaround.
@@ -779,6 +781,129 @@ __device__ __forceinline__ void zwrap_cell(const LatParams &p, const StepParams 
     }
 }
 
+// ---- two cells per thread (2-byte storage, the regularized collision)
+// The 2-byte bulk is bound by instruction issue, and half its instructions are
+// FP32 arithmetic: a compute thread takes the cells n and n + 1 (n even)
+// through the packed arithmetic of f32x2.cuh, one shared-memory word per plane
+// and direction where the plane's lead is even.  relax_fixed keeps every
+// rounding, and each cell draws the random bits it drew alone, so results are
+// the same.  us per step, one cell per thread -> pairs: 512x256x256 FP16 531 ->
+// 493, BF16 541 -> 490, 320x160x160 FP16 174 -> 145.  A fluid cell is never at the end of a row (x is not periodic), so
+// a pair that holds one lies in one row.
+template <class S> __device__ __forceinline__ F2 pair_floats(uint32_t w);
+template <> __device__ __forceinline__ F2 pair_floats<__half>(uint32_t w) { return F2(__half22float2(*reinterpret_cast<const __half2 *>(&w))); }
+template <> __device__ __forceinline__ F2 pair_floats<__nv_bfloat16>(uint32_t w) {
+    return F2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+
+template <class S, int P, int FEAT, bool RAG>
+__device__ __forceinline__ void bulk_pairs(const LatParams &p, const StepParams &s, uint8_t *buf, uint32_t n0, bool zper) {
+    constexpr uint32_t T = Tile<S>::cells, SLOT = slot_bytes<S>();
+    constexpr int SC = std::is_same<S, __half>::value ? (int)FP16_SCALE : 1;
+    const Consts<float> &k = p.kf;
+    // lead even (a pair is one word): known here unless the rows are ragged
+    auto word = [](int j) { return P == 0 || j == 0 || (!RAG && CX(j) == 0); };
+#pragma unroll 1
+    for (uint32_t c = 2 * threadIdx.x; c < T; c += 2 * Tma<S>::cthreads) {
+        const uint32_t n = n0 + c;
+        if (n >= p.N) break;
+        const uint2 fg = *reinterpret_cast<const uint2 *>(buf + 19 * SLOT + 4 * c);
+        const bool a0 = (fg.x & ~FLAG_XFACE) == 0u, a1 = (fg.y & ~FLAG_XFACE) == 0u && n + 1 < p.N;
+        if (!(a0 || a1)) continue;
+        uint32_t x, y, z;
+        coords(p, a0 ? n : n + 1, x, y, z);
+        if (!a0) x--;  // (the row of the fluid cell; it is not the row's first)
+        if (P == 1 && zper && (z == 0 || z == p.NZ - 1)) {
+            if (a0) zwrap_cell<S, 0, RAG>(p, s, buf, c, n, x, y, z);
+            if (a1) zwrap_cell<S, 0, RAG>(p, s, buf, c + 1, n + 1, x + 1, y, z);
+            continue;
+        }
+        F2 f[19];
+#pragma unroll
+        for (int i = 0; i < 19; i++) {
+            const int j = (P == 0 || i == 0) ? i : OPP(i);  // plane holding input f[i]
+            const S *q = (const S *)(buf + j * SLOT) + lead_of<S, P, RAG>(p, j) + c;
+            if (word(j)) {
+                f[i] = pair_floats<S>(*reinterpret_cast<const uint32_t *>(q));
+            } else if constexpr (SC != 1) {
+                f[i] = F2(__half2float(q[0]), __half2float(q[1]));
+            } else {
+                f[i] = F2(Pop<S>::cvt(q[0]), Pop<S>::cvt(q[1]));
+            }
+        }
+        F2 sp(0.0f);
+        if (p.sponge_on) {
+            const float *t = p.sp_tab, yz = max(__ldg(t + p.NX + y), __ldg(t + p.NX + p.NY + z));
+            sp = F2(max(__ldg(t + x), yz), max(__ldg(t + x + 1), yz));
+        }
+        relax_fixed<F2, SC, (FEAT & 2) != 0, RAG ? rf_direct<S, P>() : rf_staged<P>()>(k, moments<F2>(f), sp, f);
+        uint32_t out[19];  // per direction: cell n in the low half, n + 1 in the high half
+        Rng r0{sr_hash_mix(n, s.seed_mix)}, r1{sr_hash_mix(n + 1, s.seed_mix)};
+        const uint32_t h0 = r0.s, h1 = r1.s;
+        constexpr_for<0, 10>([&](auto kk) {
+            constexpr int K = decltype(kk)::value, i = 2 * K;
+            uint32_t b0, b1;
+            if constexpr (RAG) {
+                // the bits of a ragged lattice are the direct kernel's: one step of
+                // the sequence per value, of which the conversion takes the upper half
+                b0 = r0.next();
+                b1 = r1.next();
+                if (i + 1 < 19) {
+                    b0 = __byte_perm(b0, r0.next(), 0x7632);
+                    b1 = __byte_perm(b1, r1.next(), 0x7632);
+                }
+            } else {
+                b0 = pair_bits<K>(h0);
+                b1 = pair_bits<K>(h1);
+            }
+            if constexpr (i + 1 < 19) {
+                const uint32_t w0 = Pop<S>::rs2(f[i + 1].v.x, f[i].v.x, b0), w1 = Pop<S>::rs2(f[i + 1].v.y, f[i].v.y, b1);
+                out[i] = __byte_perm(w0, w1, 0x5410);
+                out[i + 1] = __byte_perm(w0, w1, 0x7632);
+            } else {
+                out[i] = __byte_perm(Pop<S>::rs2(f[i].v.x, 0.0f, b0), Pop<S>::rs2(f[i].v.y, 0.0f, b1), 0x7632);
+            }
+        });
+        // the plane receiving output i
+        auto dst = [&](int i) {
+            const int j = P == 0 ? OPP(i) : i;
+            return (S *)(buf + j * SLOT) + lead_of<S, P, RAG>(p, j) + c;
+        };
+        if (a0 && a1) {
+#pragma unroll
+            for (int i = 0; i < 19; i++) {
+                S *q = dst(i);
+                if (word(P == 0 ? OPP(i) : i)) {
+                    *reinterpret_cast<uint32_t *>(q) = out[i];
+                } else {
+                    q[0] = Pop<S>::bits(out[i] & 0xffffu);
+                    q[1] = Pop<S>::bits(out[i] >> 16);
+                }
+            }
+        } else if (a0) {
+#pragma unroll
+            for (int i = 0; i < 19; i++) dst(i)[0] = Pop<S>::bits(out[i] & 0xffffu);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 19; i++) dst(i)[1] = Pop<S>::bits(out[i] >> 16);
+        }
+        if ((fg.x | fg.y) & FLAG_XFACE) {
+            // (only fluid cells carry the bit; a row of four has both its cells in one pair)
+            S o[19];
+            if (a0 && (fg.x & FLAG_XFACE)) {
+#pragma unroll
+                for (int i = 0; i < 19; i++) o[i] = Pop<S>::bits(out[i] & 0xffffu);
+                xface_from_inner<S, P, RAG>(p, s, buf, c, n, x, y, z, o);
+            }
+            if (a1 && (fg.y & FLAG_XFACE)) {
+#pragma unroll
+                for (int i = 0; i < 19; i++) o[i] = Pop<S>::bits(out[i] >> 16);
+                xface_from_inner<S, P, RAG>(p, s, buf, c + 1, n + 1, x + 1, y, z, o);
+            }
+        }
+    }
+}
+
 template <class S, int P, int COLL, int FEAT, bool RAG>
 __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tma(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
     using R = typename Pop<S>::real;
@@ -885,6 +1010,9 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
         uint8_t *buf = sm + b * BUF;
         const uint32_t *fl = (const uint32_t *)(buf + 19 * SLOT);
         const uint32_t n0 = t * T;
+        if constexpr (sizeof(S) == 2 && COLL == 0 && FEAT != 0) {
+            bulk_pairs<S, P, FEAT, RAG>(p, s, buf, n0, zper);
+        } else
 #pragma unroll 1
         for (uint32_t c = threadIdx.x; c < T; c += Tma<S>::cthreads) {
             const uint32_t n = n0 + c;
@@ -925,22 +1053,12 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
                 const uint32_t h = rng.s;
                 constexpr_for<0, 10>([&](auto kk) {
                     constexpr int K = decltype(kk)::value, i = 2 * K;
-                    // the bits of a ragged lattice are the direct kernel's: one
-                    // step of the sequence per value, of which the conversion
-                    // takes the upper half
-                    uint32_t bits;
-                    if constexpr (RAG) {
-                        const uint32_t b0 = rng.next();
-                        bits = i + 1 < 19 ? __byte_perm(b0, rng.next(), 0x7632) : b0;
-                    } else {
-                        bits = pair_bits<K>(h);
-                    }
                     if constexpr (i + 1 < 19) {
-                        const uint32_t h2 = Pop<S>::rs2(f[i + 1], f[i], bits);
+                        const uint32_t h2 = Pop<S>::rs2(f[i + 1], f[i], pair_bits<K>(h));
                         out[i] = Pop<S>::bits(h2 & 0xffffu);
                         out[i + 1] = Pop<S>::bits(h2 >> 16);
                     } else {
-                        out[i] = Pop<S>::bits(Pop<S>::rs2(f[i], 0.0f, bits) >> 16);
+                        out[i] = Pop<S>::bits(Pop<S>::rs2(f[i], 0.0f, pair_bits<K>(h)) >> 16);
                     }
                 });
             } else {

@@ -7,12 +7,14 @@
 // (the direct kernel) and its compile-time form (the staged kernel), and
 // flags in V select them.
 #pragma once
+#include "f32x2.cuh"
 #include "lbm_device.cuh"
 
 namespace lbm {
 
 __device__ __forceinline__ float xfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float xmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float xmul_apart(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float xadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float xrcp(float a) { return 1.0f / a; }
 __device__ __forceinline__ float xsqrt(float a) { return sqrtf(a); }
@@ -29,6 +31,10 @@ template <int P> constexpr int rf_staged() { return RF_ODD | RF_SHIFT | (P == 0 
 // tau of a cell's sponge factor (shader.rs:832-833)
 __device__ __forceinline__ float sponge_tau(const Consts<float> &k, float sp, float tau) {
     return (sp > 0.0f && k.sponge_tau > tau) ? xfma(xmul(sp, sp), xadd(k.sponge_tau, -tau), tau) : tau;
+}
+
+__device__ __forceinline__ F2 sponge_tau(const Consts<float> &k, F2 sp, F2 tau) {
+    return F2(sponge_tau(k, sp.v.x, tau.v.x), sponge_tau(k, sp.v.y, tau.v.y));
 }
 
 // m: the moments of f in storage units (scale SC); sp: the sponge factor (0
@@ -63,7 +69,7 @@ __device__ __forceinline__ void relax_fixed(const Consts<float> &k, const Moment
     const T s3 = xadd(xadd(pxx, pyy), pzz), tr = xmul(s3, t3);
     const T bq = xfma(-rho, usq, rho1), sr = xmul(sg, rho1);
     const T left = (V & RF_USQ) ? xfma(xval<T>(-1.5f), uu, one) : xadd(one, -usq);
-    const T cb = (V & RF_SHIFT) ? xfma(-sr, left, bq) : xadd(bq, xmul(-sr, left));
+    const T cb = (V & RF_SHIFT) ? xfma(-sr, left, bq) : xadd(bq, xmul_apart(-sr, left));
     const T c0 = xadd(rho, -sr);
     const T cA = xmul(xval<T>(4.5f), c0), cO = xmul(xval<T>(3.0f), c0);
     const T wa = xval<T>((float)(SC / 18.0)), we = xval<T>((float)(SC / 36.0)), w0 = xval<T>((float)(SC / 3.0));
