@@ -1447,10 +1447,9 @@ static cudaError_t step_t(const LatParams &p, const StepParams &s0, cudaStream_t
     if (ev && ev[0]) cudaEventRecord(ev[0], st);
     if (p.moving) {
         // re-voxelize the spinning part's swept box for this step's rotation
-        // (lattice.rs:719-723): triangles -> link scratch, cells, scratch reset
+        // (lattice.rs:719-723): triangles -> link scratch, then the cells
         if (p.ntri) launch_pdl(pdl, k_tri_scatter, blocks_for((uint64_t)p.ntri * 32u), BLOCK, 0, st, p, s);
         launch_pdl(pdl, k_voxelize<S, 1 - P>, blocks_for(p.nrec), BLOCK, 0, st, p, s);
-        launch_pdl(pdl, k_qclear, blocks_for((uint64_t)p.nrec * 9u), BLOCK, 0, st, p);
     }
     const bool overlap = pdl && wb.far && p.nrec && s.nface && !p.moving;
     const bool aside = pdl && wb.side && p.nrec && !p.moving;

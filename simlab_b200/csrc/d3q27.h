@@ -84,7 +84,7 @@ struct LevelParams {
     uint32_t ntri;
     int32_t box_lo[3];
     uint32_t box_n[3];
-    uint32_t *qscr;             // 13 positive links x (nearest t, farthest t, hits) per box cell
+    uint32_t *qscr;             // two sets of 13 positive links x (nearest t, farthest t, hits) rows of box cells
     Consts27<float> kf;
     Consts27<double> kd;
 };
@@ -94,6 +94,7 @@ struct StepArgs {
     uint32_t mw;        // moment slot this step writes (mom_child)
     uint32_t mold, mnew;  // ghost fill: the parent's moment slots at the start and end of its step
     uint32_t seed_mix;  // stochastic rounding: the step seed's term of the hash
+    uint32_t scr;       // link scratch set of this finest step
     uint32_t part;      // the finest step's place among the kept block partials
     float blend;        // ghost fill: time fraction between mold and mnew
     float omega[3];     // wall angular velocity, rad per finest step

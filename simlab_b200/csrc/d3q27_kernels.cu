@@ -556,7 +556,6 @@ __device__ __forceinline__ bool wall_record(const LevelParams &p, const StepArgs
 
 template <class S>
 __global__ void __launch_bounds__(BLK, WallOcc<S>::value) k27_walls(const __grid_constant__ LevelParams p, const __grid_constant__ StepArgs a) {
-    lbm::pdl_release();
     lbm::pdl_wait();
     const uint32_t r = blockIdx.x * BLK + threadIdx.x;
     // every record's force and moment enters the step's sum (mshader.rs:519-562
@@ -572,7 +571,6 @@ __global__ void __launch_bounds__(BLK, WallOcc<S>::value) k27_walls(const __grid
 template <class S, bool FORCE, bool WRAP, bool SPONGE>
 __global__ void __launch_bounds__(BLK, StepOcc<S, WRAP, SPONGE>::value) k27_step(const __grid_constant__ LevelParams p, const StepArgs a) {
     using R = typename Pop<S>::real;
-    lbm::pdl_release();
     lbm::pdl_wait();
     const uint32_t n = blockIdx.x * BLK + threadIdx.x;
     if (n >= p.N) return;
@@ -605,7 +603,6 @@ __global__ void __launch_bounds__(BLK, StepOcc<S, WRAP, SPONGE>::value) k27_step
 template <class S>
 __global__ void __launch_bounds__(BLK) k27_face(const __grid_constant__ LevelParams p, const StepArgs a) {
     using R = typename Pop<S>::real;
-    lbm::pdl_release();
     lbm::pdl_wait();
     const uint32_t kk = blockIdx.x * BLK + threadIdx.x;
     if (kk >= p.nface) return;
@@ -651,7 +648,6 @@ __global__ void __launch_bounds__(BLK) k27_face(const __grid_constant__ LevelPar
 template <class S>
 __global__ void __launch_bounds__(BLK) k27_ghost(const __grid_constant__ LevelParams p, const StepArgs a) {
     using R = typename Pop<S>::real;
-    lbm::pdl_release();
     lbm::pdl_wait();
     const uint32_t kk = blockIdx.x * BLK + threadIdx.x;
     if (kk >= p.nghost) return;
@@ -697,7 +693,6 @@ __global__ void __launch_bounds__(BLK) k27_ghost(const __grid_constant__ LevelPa
 template <class S>
 __global__ void __launch_bounds__(BLK) k27_restrict(const __grid_constant__ LevelParams p, const StepArgs a) {
     using R = typename Pop<S>::real;
-    lbm::pdl_release();
     lbm::pdl_wait();
     const uint32_t kk = blockIdx.x * BLK + threadIdx.x;
     if (kk >= p.nrestrict) return;
@@ -859,11 +854,12 @@ __device__ __forceinline__ bool solid(const LevelParams &p, const float *rot, in
 __device__ __forceinline__ bool in_box(const LevelParams &p, int lx, int ly, int lz) {
     return lx >= 0 && ly >= 0 && lz >= 0 && lx < (int)p.box_n[0] && ly < (int)p.box_n[1] && lz < (int)p.box_n[2];
 }
+// the link scratch as lbm::rv::link_scratch lays it out, 13 links a set
+__device__ __forceinline__ uint32_t *link_scratch(const LevelParams &p, uint32_t set) { return p.qscr + (uint64_t)set * 39u * p.nrec; }
 }  // namespace sp27
 
 __global__ void __launch_bounds__(BLK) k27_tri_scatter(const __grid_constant__ LevelParams p, const StepArgs a) {
     using namespace lbm::rv;
-    lbm::pdl_release();
     lbm::pdl_wait();
     // one warp per triangle, its lanes over the lattice points near it
     const uint32_t t = (blockIdx.x * BLK + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
@@ -888,6 +884,7 @@ __global__ void __launch_bounds__(BLK) k27_tri_scatter(const __grid_constant__ L
     }
     const int nx = hi[0] - lo[0] + 1, ny = hi[1] - lo[1] + 1, nz = hi[2] - lo[2] + 1;
     const int npts = (nx > 0 && ny > 0 && nz > 0) ? nx * ny * nz : 0;
+    uint32_t *scr = sp27::link_scratch(p, a.scr);
     for (int q = (int)lane; q < npts; q += 32) {
                 const int x = lo[0] + q % nx, y = lo[1] + (q / nx) % ny, z = lo[2] + q / (nx * ny);
                 const V3 pt = {(float)x, (float)y, (float)z};
@@ -901,34 +898,27 @@ __global__ void __launch_bounds__(BLK) k27_tri_scatter(const __grid_constant__ L
                     if (fm(d0, d1) > 0.0f && fabsf(d0) > 1e-6f) continue;
                     const float tt = ray_tri(pt, cv, va, e1, e2);
                     if (tt <= 1.0f) {
-                        const uint64_t o = ((uint64_t)k * 13u + (uint32_t)(i - 14)) * 3u;
+                        uint32_t *q0 = scr + (uint64_t)(3 * (i - 14)) * p.nrec + k;
                         const uint32_t tb = __float_as_uint(tt > 0.0f ? tt : 0.0f);
-                        atomicMin(p.qscr + o, tb);
-                        atomicMax(p.qscr + o + 1, tb);
-                        atomicAdd(p.qscr + o + 2, 1u);
+                        atomicMin(q0, tb);
+                        atomicMax(q0 + p.nrec, tb);
+                        atomicAdd(q0 + 2ull * p.nrec, 1u);
                     }
                 }
             }
-}
-
-__global__ void __launch_bounds__(BLK) k27_qclear(const __grid_constant__ LevelParams p) {
-    lbm::pdl_release();
-    lbm::pdl_wait();
-    const uint64_t k = (uint64_t)blockIdx.x * BLK + threadIdx.x;
-    if (k >= (uint64_t)p.nrec * 13u) return;
-    p.qscr[3 * k] = 0x7f7fffffu;
-    p.qscr[3 * k + 1] = 0u;
-    p.qscr[3 * k + 2] = 0u;
 }
 
 template <class S>
 __global__ void __launch_bounds__(BLK) k27_voxelize(const __grid_constant__ LevelParams p, const StepArgs a) {
     using namespace lbm::rv;
     using R = typename Pop<S>::real;
-    lbm::pdl_release();
     lbm::pdl_wait();
     const uint32_t k = blockIdx.x * BLK + threadIdx.x;
     if (k >= p.nrec) return;
+    // the other scratch set, read by the step before, is reset for the next one
+    uint32_t *scr = sp27::link_scratch(p, a.scr), *next = sp27::link_scratch(p, a.scr ^ 1u);
+#pragma unroll
+    for (int w = 0; w < 39; w++) next[(uint64_t)w * p.nrec + k] = w % 3 == 0 ? 0x7f7fffffu : 0u;
     const int lx = (int)(k % p.box_n[0]), ly = (int)((k / p.box_n[0]) % p.box_n[1]), lz = (int)(k / (p.box_n[0] * p.box_n[1]));
     const int px = lx + p.box_lo[0], py = ly + p.box_lo[1], pz = lz + p.box_lo[2];
     const uint32_t n = ((uint32_t)pz * p.NY + (uint32_t)py) * p.NX + (uint32_t)px;
@@ -954,14 +944,14 @@ __global__ void __launch_bounds__(BLK) k27_voxelize(const __grid_constant__ Leve
             qv[i] = 9.0f; qx[i] = -1.0f; nh[i] = 0u;
             if (i == 13) continue;
             if (i > 13) {
-                const uint64_t o = ((uint64_t)k * 13u + (uint32_t)(i - 14)) * 3u;
-                const uint32_t c = p.qscr[o + 2];
-                if (c) { qv[i] = __uint_as_float(p.qscr[o]); qx[i] = __uint_as_float(p.qscr[o + 1]); nh[i] = c; }
+                const uint32_t *q0 = scr + (uint64_t)(3 * (i - 14)) * p.nrec + k;
+                const uint32_t c = q0[2ull * p.nrec], v0 = q0[0], v1 = q0[p.nrec];
+                if (c) { qv[i] = __uint_as_float(v0); qx[i] = __uint_as_float(v1); nh[i] = c; }
             } else if (sp27::in_box(p, lx + CX(i), ly + CY(i), lz + CZ(i))) {
                 const uint32_t k2 = ((uint32_t)(lz + CZ(i)) * p.box_n[1] + (uint32_t)(ly + CY(i))) * p.box_n[0] + (uint32_t)(lx + CX(i));
-                const uint64_t o = ((uint64_t)k2 * 13u + (uint32_t)(26 - i - 14)) * 3u;
-                const uint32_t c = p.qscr[o + 2];
-                if (c) { qv[i] = fs(1.0f, __uint_as_float(p.qscr[o + 1])); qx[i] = fs(1.0f, __uint_as_float(p.qscr[o])); nh[i] = c; }
+                const uint32_t *q0 = scr + (uint64_t)(3 * (26 - i - 14)) * p.nrec + k2;
+                const uint32_t c = q0[2ull * p.nrec], v0 = q0[0], v1 = q0[p.nrec];
+                if (c) { qv[i] = fs(1.0f, __uint_as_float(v1)); qx[i] = fs(1.0f, __uint_as_float(v0)); nh[i] = c; }
             }
         }
         uint32_t mask = 0;
@@ -1166,7 +1156,6 @@ cudaError_t launch27_revoxel(int storage, const LevelParams &p, const StepArgs &
         return cudaGetLastError();
     });
     if (e != cudaSuccess) return e;
-    lbm::launch_pdl(true, k27_qclear, blocks_for((uint64_t)p.nrec * 13u), BLK, 0, st, p);
     return cudaGetLastError();
 }
 

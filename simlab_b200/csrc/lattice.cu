@@ -72,6 +72,7 @@ struct lbm_lattice {
     lbm::LatParams lp{};
     cudaStream_t stream = nullptr;
     lbm::WallsBeside walls_beside;
+    uint32_t scr = 0;        // link scratch set of the next step (the other is being reset)
     uint32_t ring = 1;       // steps whose wall-kernel partials are kept before they are summed
     int device = 0;
     std::vector<void *> allocs;
@@ -205,6 +206,7 @@ lbm::StepParams step_params(const lbm_lattice *h, const lbm_step_in &s, uint32_t
     sp.next_seed_mix = ((uint32_t)(step_index + 1) * lbm::STEP_SEED_MUL) * 0x85EBCA77u + 0x632BE5ABu;
     sp.nface = h->fused_valid ? h->nface_rest : h->nface;
     sp.part = slot % h->ring;
+    sp.scr = h->scr;
     for (int a = 0; a < 3; a++) {
         sp.omega[a] = (float)s.omega[a];
         sp.omega_d[a] = s.omega[a];
@@ -584,8 +586,9 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
         p.ntri = (uint32_t)spin->ntri;
         p.tris = (const float4 *)h->dalloc(std::max<uint64_t>(spin->ntri, 1) * 48);
         if (spin->ntri) ck(cudaMemcpy((void *)p.tris, spin->tris, spin->ntri * 48, cudaMemcpyHostToDevice), "upload triangles");
-        std::vector<uint32_t> q0((size_t)nrec * 27, 0u);
-        for (size_t k = 0; k < q0.size(); k += 3) q0[k] = 0x7f7fffffu;  // nearest hit: FLT_MAX
+        std::vector<uint32_t> q0((size_t)nrec * 54, 0u);
+        for (size_t w = 0; w < 54; w += 3)
+            std::fill_n(q0.begin() + (ptrdiff_t)(w * nrec), nrec, 0x7f7fffffu);  // nearest hit: FLT_MAX
         p.qscr = (uint32_t *)h->dalloc(q0.size() * 4);
         ck(cudaMemcpy(p.qscr, q0.data(), q0.size() * 4, cudaMemcpyHostToDevice), "upload link scratch");
     }
@@ -689,7 +692,7 @@ void run_impl(lbm_lattice *h, const lbm_step_in *steps, uint64_t n, double *forc
                 }
                 h->prof_steps++;
                 // the kernels launch_step enqueues for this step
-                h->prof_launches += (sp.nface ? 1u : 0u) + (p.nrec ? 1u : 0u) + 1u + (p.moving ? 2u + (p.ntri ? 1u : 0u) : 0u);
+                h->prof_launches += (sp.nface ? 1u : 0u) + (p.nrec ? 1u : 0u) + 1u + (p.moving ? 1u + (p.ntri ? 1u : 0u) : 0u);
                 if (si.sample) h->prof_launches += (h->nvert ? 1u : 0u) + (h->npix ? 1u : 0u);
             }
             ck(lbm::launch_step(h->setup.storage, p, sp, (int)(idx % 2), h->setup.collision, h->stream, h->walls_beside, evs),
@@ -699,6 +702,7 @@ void run_impl(lbm_lattice *h, const lbm_step_in *steps, uint64_t n, double *forc
                                       h->nslices, h->npix, h->sacc, h->stream),
                    "sample kernels");
             h->steps_done++;
+            h->scr ^= 1u;
             h->fused_valid = h->xfuse;
             if (p.nrec && ((k + 1) % h->ring == 0 || k + 1 == len))
                 ck(lbm::launch_force_sum(p, k - k % h->ring, k % h->ring + 1, h->stream), "force sum");

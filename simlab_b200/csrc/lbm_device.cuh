@@ -161,7 +161,7 @@ struct LatParams {
     uint32_t ntri;
     int32_t box_lo[3];
     uint32_t box_n[3];
-    uint32_t *qscr;            // 9 links x (nearest t, farthest t, hits) per box cell
+    uint32_t *qscr;            // two sets of 9 links x (nearest t, farthest t, hits) rows of box cells
     Consts<float> kf;
     Consts<double> kd;
 };
@@ -172,6 +172,7 @@ struct StepParams {
     uint32_t next_seed_mix;  // the same for the next step
     uint32_t nface;          // face cells the face kernel handles this step
     uint32_t part;   // the step's place among the kept block partials
+    uint32_t scr;    // link scratch set of this step
     int beside;      // this kernel runs beside the wall kernel, not after it
     float omega[3];  // angular velocity, rad per step
     double omega_d[3];

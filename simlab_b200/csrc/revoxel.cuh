@@ -5,8 +5,8 @@
 // cell of the swept box is classified (k_voxelize): solid or fluid from the
 // body-frame occupancy grid, cut links and q from the scratch, a refill of
 // the populations a just-uncovered cell would have sent out, and the momentum
-// the part takes from cells it covers or gives to cells it uncovers; finally
-// the scratch is reset for the next step (k_qclear).
+// the part takes from cells it covers or gives to cells it uncovers; it
+// also resets the scratch of the next step.
 //
 // The geometric arithmetic is f32 rounded operation by operation (no fused
 // multiply-add, IEEE division and square root), as the reference states it,
@@ -30,12 +30,18 @@ __device__ __forceinline__ bool solid_at(const LatParams &p, const StepParams &s
     return occ_at(p, to_body(before ? s.rot_prev : s.rot, pc));
 }
 
+// The link scratch: per set, 9 links x (nearest t, farthest t, hits), each a
+// row of one word per box cell, so that a warp's cells read whole sectors (by
+// cell, 27 words apart, every load touched 32 of them).  Two sets take turns:
+// k_voxelize reads one and resets the other (shader.rs:942-948).  256x128x128
+// rotor, 113 k box cells: k_voxelize 44 us and a reset kernel before, 24 us.
+__device__ __forceinline__ uint32_t *link_scratch(const LatParams &p, uint32_t set) { return p.qscr + (uint64_t)set * 27u * p.nrec; }
+
 }  // namespace rv
 
 // shader.rs:902-940: one thread per triangle
 __global__ void __launch_bounds__(BLOCK) k_tri_scatter(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
     using namespace rv;
-    pdl_release();
     pdl_wait();
     // one warp per triangle, its lanes over the lattice points near it
     const uint32_t t = (blockIdx.x * BLOCK + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
@@ -58,6 +64,7 @@ __global__ void __launch_bounds__(BLOCK) k_tri_scatter(const __grid_constant__ L
                        min((int)floorf(fa(fmaxf(fmaxf(a.z, b.z), c.z), 1.415f)), p.box_lo[2] + (int)p.box_n[2] - 1)};
     const int nx = hi[0] - lo[0] + 1, ny = hi[1] - lo[1] + 1, nz = hi[2] - lo[2] + 1;
     const int npts = (nx > 0 && ny > 0 && nz > 0) ? nx * ny * nz : 0;
+    uint32_t *scr = link_scratch(p, s.scr);
     for (int q = (int)lane; q < npts; q += 32) {
                 const int x = lo[0] + q % nx, y = lo[1] + (q / nx) % ny, z = lo[2] + q / (nx * ny);
                 const V3 pt = {(float)x, (float)y, (float)z};
@@ -71,25 +78,14 @@ __global__ void __launch_bounds__(BLOCK) k_tri_scatter(const __grid_constant__ L
                     if (fm(d0, d1) > 0.0f && fabsf(d0) > 1e-6f) continue;
                     const float tt = ray_tri(pt, cv, a, e1, e2);
                     if (tt <= 1.0f) {
-                        const uint64_t o = ((uint64_t)k * 9u + (uint32_t)(i - 1) / 2u) * 3u;
+                        uint32_t *q0 = scr + (uint64_t)(3 * ((i - 1) / 2)) * p.nrec + k;
                         const uint32_t tb = __float_as_uint(tt > 0.0f ? tt : 0.0f);
-                        atomicMin(p.qscr + o, tb);
-                        atomicMax(p.qscr + o + 1, tb);
-                        atomicAdd(p.qscr + o + 2, 1u);
+                        atomicMin(q0, tb);
+                        atomicMax(q0 + p.nrec, tb);
+                        atomicAdd(q0 + 2ull * p.nrec, 1u);
                     }
                 }
             }
-}
-
-// shader.rs:942-948
-__global__ void __launch_bounds__(BLOCK) k_qclear(const __grid_constant__ LatParams p) {
-    pdl_release();
-    pdl_wait();
-    const uint64_t k = (uint64_t)blockIdx.x * BLOCK + threadIdx.x;
-    if (k >= (uint64_t)p.nrec * 9u) return;
-    p.qscr[3 * k] = 0x7f7fffffu;
-    p.qscr[3 * k + 1] = 0u;
-    p.qscr[3 * k + 2] = 0u;
 }
 
 // shader.rs:953-1104: one thread per swept-box cell (record k); Q is the
@@ -99,10 +95,13 @@ template <class S, int Q>
 __global__ void __launch_bounds__(BLOCK) k_voxelize(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
     using namespace rv;
     using R = typename Pop<S>::real;
-    pdl_release();
     pdl_wait();
     const uint32_t k = blockIdx.x * BLOCK + threadIdx.x;
     if (k >= p.nrec) return;
+    // the other set, read by the step before, is reset for the next one
+    uint32_t *scr = link_scratch(p, s.scr), *next = link_scratch(p, s.scr ^ 1u);
+#pragma unroll
+    for (int w = 0; w < 27; w++) next[(uint64_t)w * p.nrec + k] = w % 3 == 0 ? 0x7f7fffffu : 0u;
     const uint32_t lx = k % p.box_n[0], ly = (k / p.box_n[0]) % p.box_n[1], lz = k / (p.box_n[0] * p.box_n[1]);
     const int px = (int)lx + p.box_lo[0], py = (int)ly + p.box_lo[1], pz = (int)lz + p.box_lo[2];
     const uint32_t n = ((uint32_t)pz * p.NY + (uint32_t)py) * p.NX + (uint32_t)px;
@@ -131,16 +130,16 @@ __global__ void __launch_bounds__(BLOCK) k_voxelize(const __grid_constant__ LatP
     for (int i = 1; i < 19; i++) {
         qv[i] = 9.0f; qx[i] = -1.0f; nh[i] = 0u;
         if (i & 1) {
-            const uint64_t o = ((uint64_t)k * 9u + (uint32_t)(i - 1) / 2u) * 3u;
-            const uint32_t c = p.qscr[o + 2];
-            if (c) { qv[i] = __uint_as_float(p.qscr[o]); qx[i] = __uint_as_float(p.qscr[o + 1]); nh[i] = c; }
+            const uint32_t *q0 = scr + (uint64_t)(3 * ((i - 1) / 2)) * p.nrec + k;
+            const uint32_t c = q0[2ull * p.nrec], v0 = q0[0], v1 = q0[p.nrec];
+            if (c) { qv[i] = __uint_as_float(v0); qx[i] = __uint_as_float(v1); nh[i] = c; }
         } else {
             const int qxl = (int)lx + CX(i), qyl = (int)ly + CY(i), qzl = (int)lz + CZ(i);
             if (qxl >= 0 && qyl >= 0 && qzl >= 0 && qxl < (int)p.box_n[0] && qyl < (int)p.box_n[1] && qzl < (int)p.box_n[2]) {
                 const uint32_t k2 = ((uint32_t)qzl * p.box_n[1] + (uint32_t)qyl) * p.box_n[0] + (uint32_t)qxl;
-                const uint64_t o = ((uint64_t)k2 * 9u + (uint32_t)(i - 2) / 2u) * 3u;
-                const uint32_t c = p.qscr[o + 2];
-                if (c) { qv[i] = fs(1.0f, __uint_as_float(p.qscr[o + 1])); qx[i] = fs(1.0f, __uint_as_float(p.qscr[o])); nh[i] = c; }
+                const uint32_t *q0 = scr + (uint64_t)(3 * ((i - 2) / 2)) * p.nrec + k2;
+                const uint32_t c = q0[2ull * p.nrec], v0 = q0[0], v1 = q0[p.nrec];
+                if (c) { qv[i] = fs(1.0f, __uint_as_float(v1)); qx[i] = fs(1.0f, __uint_as_float(v0)); nh[i] = c; }
             }
         }
     }
