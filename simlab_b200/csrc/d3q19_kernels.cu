@@ -1154,16 +1154,33 @@ __device__ __forceinline__ void wall_links(const LatParams &p, const StepParams 
 // step's force and moment (plus what a spinning part's re-voxelizer booked).
 template <class R>
 __device__ __forceinline__ void record_after(const LatParams &p, uint32_t r, const R *f, R rho, R ux, R uy, R uz, R *Fo, R *To) {
-#pragma unroll
-    for (int i = 1; i < 19; i++) Rec<R>::set_fpost(p, r, i, f[i]);
-    Rec<R>::set_macro(p, r, 0, rho);
-    Rec<R>::set_macro(p, r, 1, ux);
-    Rec<R>::set_macro(p, r, 2, uy);
-    Rec<R>::set_macro(p, r, 3, uz);
     if (p.moving) {
         for (int a = 0; a < 3; a++) { Fo[a] += Rec<R>::ft(p, r, a); To[a] += Rec<R>::ft(p, r, 3 + a); }
     }
-    for (int a = 0; a < 3; a++) { Rec<R>::set_ft(p, r, a, Fo[a]); Rec<R>::set_ft(p, r, 3 + a, To[a]); }
+    if constexpr (sizeof(R) == 8) {
+#pragma unroll
+        for (int i = 1; i < 19; i++) Rec<R>::set_fpost(p, r, i, f[i]);
+        Rec<R>::set_macro(p, r, 0, rho);
+        Rec<R>::set_macro(p, r, 1, ux);
+        Rec<R>::set_macro(p, r, 2, uy);
+        Rec<R>::set_macro(p, r, 3, uz);
+        for (int a = 0; a < 3; a++) { Rec<R>::set_ft(p, r, a, Fo[a]); Rec<R>::set_ft(p, r, 3 + a, To[a]); }
+    } else {
+        // words 11..39 in 16-byte pieces: word by word, each store of a warp
+        // touched 32 sectors
+        static_assert(R_FPOST == 11 && R_MACRO == 29 && R_FT == 33 && RS == 40, "record in 16-byte pieces");
+        float w[29];
+#pragma unroll
+        for (int i = 1; i < 19; i++) w[i - 1] = f[i];
+        w[18] = rho; w[19] = ux; w[20] = uy; w[21] = uz;
+#pragma unroll
+        for (int a = 0; a < 3; a++) { w[22 + a] = Fo[a]; w[25 + a] = To[a]; }
+        w[28] = 0.0f;  // the record's spare word
+        float *rec = reinterpret_cast<float *>(p.recs + (uint64_t)r * RS);
+        rec[R_FPOST] = w[0];
+#pragma unroll
+        for (int q = 0; q < 7; q++) reinterpret_cast<float4 *>(rec)[3 + q] = make_float4(w[1 + 4 * q], w[2 + 4 * q], w[3 + 4 * q], w[4 + 4 * q]);
+    }
 }
 
 template <class S, int P, int COLL>
@@ -1447,8 +1464,9 @@ static cudaError_t step_t(const LatParams &p, const StepParams &s0, cudaStream_t
     if (ev && ev[0]) cudaEventRecord(ev[0], st);
     if (p.moving) {
         // re-voxelize the spinning part's swept box for this step's rotation
-        // (lattice.rs:719-723): triangles -> link scratch, then the cells
-        if (p.ntri) launch_pdl(pdl, k_tri_scatter, blocks_for((uint64_t)p.ntri * 32u), BLOCK, 0, st, p, s);
+        // (lattice.rs:719-723): triangles -> link scratch and solid cells, then the box
+        const uint64_t halo = ((uint64_t)p.box_n[0] + 2) * (p.box_n[1] + 2) * (p.box_n[2] + 2);
+        launch_pdl(pdl, k_tri_scatter, blocks_for((uint64_t)p.ntri * 32u) + blocks_for(halo), BLOCK, 0, st, p, s);
         launch_pdl(pdl, k_voxelize<S, 1 - P>, blocks_for(p.nrec), BLOCK, 0, st, p, s);
     }
     const bool overlap = pdl && wb.far && p.nrec && s.nface && !p.moving;

@@ -84,6 +84,7 @@ struct LevelParams {
     uint32_t ntri;
     int32_t box_lo[3];
     uint32_t box_n[3];
+    uint8_t *sol;               // per cell of the box and the layer around it: solid now (1), before (2)
     uint32_t *qscr;             // two sets of 13 positive links x (nearest t, farthest t, hits) rows of box cells
     Consts27<float> kf;
     Consts27<double> kd;

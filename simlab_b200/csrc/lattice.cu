@@ -590,6 +590,7 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
         for (size_t w = 0; w < 54; w += 3)
             std::fill_n(q0.begin() + (ptrdiff_t)(w * nrec), nrec, 0x7f7fffffu);  // nearest hit: FLT_MAX
         p.qscr = (uint32_t *)h->dalloc(q0.size() * 4);
+        p.sol = (uint8_t *)h->dalloc(((uint64_t)spin->box_n[0] + 2) * (spin->box_n[1] + 2) * (spin->box_n[2] + 2));
         ck(cudaMemcpy(p.qscr, q0.data(), q0.size() * 4, cudaMemcpyHostToDevice), "upload link scratch");
     }
     fill_consts<float>(p.kf, st);
@@ -692,7 +693,7 @@ void run_impl(lbm_lattice *h, const lbm_step_in *steps, uint64_t n, double *forc
                 }
                 h->prof_steps++;
                 // the kernels launch_step enqueues for this step
-                h->prof_launches += (sp.nface ? 1u : 0u) + (p.nrec ? 1u : 0u) + 1u + (p.moving ? 1u + (p.ntri ? 1u : 0u) : 0u);
+                h->prof_launches += (sp.nface ? 1u : 0u) + (p.nrec ? 1u : 0u) + 1u + (p.moving ? 2u : 0u);
                 if (si.sample) h->prof_launches += (h->nvert ? 1u : 0u) + (h->npix ? 1u : 0u);
             }
             ck(lbm::launch_step(h->setup.storage, p, sp, (int)(idx % 2), h->setup.collision, h->stream, h->walls_beside, evs),

@@ -161,6 +161,7 @@ struct LatParams {
     uint32_t ntri;
     int32_t box_lo[3];
     uint32_t box_n[3];
+    uint8_t *sol;              // per cell of the box and the layer around it: solid now (1), before (2)
     uint32_t *qscr;            // two sets of 9 links x (nearest t, farthest t, hits) rows of box cells
     Consts<float> kf;
     Consts<double> kd;

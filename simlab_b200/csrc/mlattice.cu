@@ -603,6 +603,7 @@ void create_multi(const lbm_multi_setup *setup, const lbm_geometry *geom, const 
         for (size_t w = 0; w < 78; w += 3)
             std::fill_n(q0.begin() + (ptrdiff_t)(w * h->nrec), h->nrec, 0x7f7fffffu);  // nearest hit: FLT_MAX
         p.qscr = (uint32_t *)h->dalloc(q0.size() * 4);
+        p.sol = (uint8_t *)h->dalloc(((uint64_t)spin->box_n[0] + 2) * (spin->box_n[1] + 2) * (spin->box_n[2] + 2));
         ck(cudaMemcpy(p.qscr, q0.data(), q0.size() * 4, cudaMemcpyHostToDevice), "upload link scratch");
     }
     for (size_t l = 0; l < nl; l++) {

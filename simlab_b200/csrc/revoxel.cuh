@@ -37,6 +37,20 @@ __device__ __forceinline__ bool solid_at(const LatParams &p, const StepParams &s
 // rotor, 113 k box cells: k_voxelize 44 us and a reset kernel before, 24 us.
 __device__ __forceinline__ uint32_t *link_scratch(const LatParams &p, uint32_t set) { return p.qscr + (uint64_t)set * 27u * p.nrec; }
 
+// Whether the cells of the swept box and the layer around it are solid now
+// (bit 0) and were before (bit 1): one byte per cell, written beside the
+// triangle scatter, so that k_voxelize looks its neighbours up instead of
+// rotating each into the body frame again (18 times a cell).
+__device__ __forceinline__ uint32_t solid_index(const uint32_t *box_n, int lx, int ly, int lz) {
+    return ((uint32_t)(lz + 1) * (box_n[1] + 2u) + (uint32_t)(ly + 1)) * (box_n[0] + 2u) + (uint32_t)(lx + 1);
+}
+__device__ __forceinline__ void solid_cell(const LatParams &p, const StepParams &s, uint32_t q) {
+    const uint32_t nx = p.box_n[0] + 2u, ny = p.box_n[1] + 2u, nz = p.box_n[2] + 2u;
+    if (q >= nx * ny * nz) return;
+    const int x = (int)(q % nx) - 1 + p.box_lo[0], y = (int)(q / nx % ny) - 1 + p.box_lo[1], z = (int)(q / (nx * ny)) - 1 + p.box_lo[2];
+    p.sol[q] = (uint8_t)((solid_at(p, s, x, y, z, false) ? 1 : 0) | (solid_at(p, s, x, y, z, true) ? 2 : 0));
+}
+
 }  // namespace rv
 
 // shader.rs:902-940: one thread per triangle
@@ -44,6 +58,12 @@ __global__ void __launch_bounds__(BLOCK) k_tri_scatter(const __grid_constant__ L
     using namespace rv;
     pdl_wait();
     // one warp per triangle, its lanes over the lattice points near it
+    // (the blocks past the triangles' classify the box's cells)
+    const uint32_t tri_blocks = (p.ntri * 32u + BLOCK - 1) / BLOCK;
+    if (blockIdx.x >= tri_blocks) {
+        solid_cell(p, s, (blockIdx.x - tri_blocks) * BLOCK + threadIdx.x);
+        return;
+    }
     const uint32_t t = (blockIdx.x * BLOCK + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
     if (t >= p.ntri) return;
     const float4 t0 = p.tris[3 * t], t1 = p.tris[3 * t + 1], t2 = p.tris[3 * t + 2];
@@ -96,19 +116,74 @@ __global__ void __launch_bounds__(BLOCK) k_voxelize(const __grid_constant__ LatP
     using namespace rv;
     using R = typename Pop<S>::real;
     pdl_wait();
-    const uint32_t k = blockIdx.x * BLOCK + threadIdx.x;
-    if (k >= p.nrec) return;
+    const uint32_t k0 = blockIdx.x * BLOCK + threadIdx.x;
+    const bool live = k0 < p.nrec;
+    const uint32_t k = live ? k0 : p.nrec - 1;  // (idle threads only help their warp)
     // the other set, read by the step before, is reset for the next one
     uint32_t *scr = link_scratch(p, s.scr), *next = link_scratch(p, s.scr ^ 1u);
 #pragma unroll
-    for (int w = 0; w < 27; w++) next[(uint64_t)w * p.nrec + k] = w % 3 == 0 ? 0x7f7fffffu : 0u;
+    for (int w = 0; w < 27; w++)
+        if (live) next[(uint64_t)w * p.nrec + k] = w % 3 == 0 ? 0x7f7fffffu : 0u;
     const uint32_t lx = k % p.box_n[0], ly = (k / p.box_n[0]) % p.box_n[1], lz = k / (p.box_n[0] * p.box_n[1]);
     const int px = (int)lx + p.box_lo[0], py = (int)ly + p.box_lo[1], pz = (int)lz + p.box_lo[2];
     const uint32_t n = ((uint32_t)pz * p.NY + (uint32_t)py) * p.NX + (uint32_t)px;
     const Consts<R> &kk = K<R>(p);
     const R pc[3] = {(R)px - kk.center[0], (R)py - kk.center[1], (R)pz - kk.center[2]};
-    const bool solid_now = solid_at(p, s, px, py, pz, false);
-    const bool solid_before = solid_at(p, s, px, py, pz, true);
+    const uint32_t sq = solid_index(p.box_n, (int)lx, (int)ly, (int)lz);
+    const bool solid_now = (p.sol[sq] & 1u) != 0, solid_before = (p.sol[sq] & 2u) != 0;
+    // Refill of the cells uncovered this step: the density and the mean
+    // non-equilibrium stress of the neighbours that are fluid now and were
+    // before.  Few cells need it, but one thread walking its 18 neighbours (two
+    // occupancy tests and a record each, one after another) took most of the
+    // kernel's time: the warp takes one such cell at a time, a lane per
+    // neighbour, and the lanes' terms are added in the neighbours' order.
+    // 256x128x128 rotor: 45 -> 16 us.
+    R rs = 0, cnt = 0, pis[6] = {0, 0, 0, 0, 0, 0};
+    const bool refill = live && !solid_now && solid_before;
+    for (uint32_t todo = __ballot_sync(0xffffffffu, refill); todo; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1, lane = (int)(threadIdx.x & 31u), i = lane + 1;
+        const int ax = __shfl_sync(0xffffffffu, px, src), ay = __shfl_sync(0xffffffffu, py, src), az = __shfl_sync(0xffffffffu, pz, src);
+        bool ok = false;
+        R t[7] = {0, 0, 0, 0, 0, 0, 0};
+        if (lane < 18) {
+            const int nx = ax + CX(i), ny = ay + CY(i), nz = az + CZ(i);
+            const int qxl = nx - p.box_lo[0], qyl = ny - p.box_lo[1], qzl = nz - p.box_lo[2];
+            ok = p.sol[solid_index(p.box_n, qxl, qyl, qzl)] == 0 && qxl >= 0 && qyl >= 0 && qzl >= 0 && qxl < (int)p.box_n[0] && qyl < (int)p.box_n[1] &&
+                 qzl < (int)p.box_n[2];
+            if (ok) {
+                const uint32_t k2 = ((uint32_t)qzl * p.box_n[1] + (uint32_t)qyl) * p.box_n[0] + (uint32_t)qxl;
+                R fp[19];
+                fp[0] = 0;
+                for (int j = 1; j < 19; j++) fp[j] = Rec<R>::fpost(p, k2, j);
+                const Moments<R> m2 = moments<R>(fp);
+                const R r2 = Rec<R>::macro(p, k2, 0);
+                const R u2[3] = {Rec<R>::macro(p, k2, 1), Rec<R>::macro(p, k2, 2), Rec<R>::macro(p, k2, 3)};
+                const R tr = (m2.sxx + m2.syy + m2.szz) / (R)3;
+                const R uu = u2[0] * u2[0] + u2[1] * u2[1] + u2[2] * u2[2];
+                t[0] = m2.sxx - tr - r2 * (u2[0] * u2[0] - uu / (R)3);
+                t[1] = m2.syy - tr - r2 * (u2[1] * u2[1] - uu / (R)3);
+                t[2] = m2.szz - tr - r2 * (u2[2] * u2[2] - uu / (R)3);
+                t[3] = m2.sxy - r2 * u2[0] * u2[1];
+                t[4] = m2.sxz - r2 * u2[0] * u2[2];
+                t[5] = m2.syz - r2 * u2[1] * u2[2];
+                t[6] = r2;
+            }
+        }
+        const uint32_t use = __ballot_sync(0xffffffffu, ok);
+        for (int q = 0; q < 18; q++) {
+            if (!(use >> q & 1u)) continue;
+            R v[7];
+#pragma unroll
+            for (int j = 0; j < 7; j++) v[j] = __shfl_sync(0xffffffffu, t[j], q);
+            if (lane == src) {
+                rs += v[6];
+                cnt += (R)1;
+#pragma unroll
+                for (int j = 0; j < 6; j++) pis[j] += v[j];
+            }
+        }
+    }
+    if (!live) return;
     R F[3] = {0, 0, 0};
     if (solid_now) {
         p.flags[n] = 1u | ((k + 1u) << 2);
@@ -143,12 +218,17 @@ __global__ void __launch_bounds__(BLOCK) k_voxelize(const __grid_constant__ LatP
             }
         }
     }
-    uint32_t mask = 0;
+    uint32_t mask = 0, near = 0;  // near: the solid neighbours
+    {
+        const int sx = (int)p.box_n[0] + 2, sxy = sx * ((int)p.box_n[1] + 2);
+#pragma unroll
+        for (int i = 1; i < 19; i++) near |= (p.sol[(int)sq + CX(i) + CY(i) * sx + CZ(i) * sxy] & 1u) << i;
+    }
 #pragma unroll
     for (int i = 1; i < 19; i++) {
         // a wall where the neighbour is solid, or where the link crosses a
         // sheet thinner than a cell (two hits); q from the nearest hit
-        if (solid_at(p, s, px + CX(i), py + CY(i), pz + CZ(i), false)) {
+        if (near & (1u << i)) {
             if (nh[i] == 0u) qv[i] = 1.0f;
             mask |= 1u << i;
         } else if (nh[i] >= 2u && fs(qx[i], qv[i]) > 1e-5f) {
@@ -157,43 +237,30 @@ __global__ void __launch_bounds__(BLOCK) k_voxelize(const __grid_constant__ LatP
             qv[i] = 1.0f;
         }
     }
+    // the record's first words in 16-byte pieces (mask, cell, distances; word 11
+    // starts the populations)
+    static_assert(RS * 4 % 16 == 0 && R_MASK == 0 && R_CELL == 1 && R_Q == 2 && R_FPOST == 11 && R_FT == 33, "record in 16-byte pieces");
+    uint32_t qw[11];
+    qw[0] = mask;
+    qw[1] = n;
 #pragma unroll
     for (int w = 0; w < 9; w++) {
         const uint32_t lo = __half_as_ushort(__float2half_rn(fminf(qv[2 * w + 1], 1.0f)));
         const uint32_t hi = __half_as_ushort(__float2half_rn(fminf(qv[2 * w + 2], 1.0f)));
-        p.recs[k * RS + R_Q + w] = lo | (hi << 16);
+        qw[R_Q + w] = lo | (hi << 16);
     }
-    p.recs[k * RS + R_MASK] = mask;
+    {
+        uint32_t *rec = p.recs + (uint64_t)k * RS;
+        reinterpret_cast<uint4 *>(rec)[0] = make_uint4(qw[0], qw[1], qw[2], qw[3]);
+        reinterpret_cast<uint4 *>(rec)[1] = make_uint4(qw[4], qw[5], qw[6], qw[7]);
+        reinterpret_cast<uint2 *>(rec)[4] = make_uint2(qw[8], qw[9]);
+        rec[10] = qw[10];
+    }
     if (solid_before) {
         // uncovered this step: refill what the cell would have sent out last
         // step, the equilibrium at the wall velocity and the density of the
-        // fluid neighbours plus their mean non-equilibrium stress; the part
-        // gives up the refill's momentum
-        R rs = 0, cnt = 0, pis[6] = {0, 0, 0, 0, 0, 0};
-        for (int i = 1; i < 19; i++) {
-            const bool fluid_now = !solid_at(p, s, px + CX(i), py + CY(i), pz + CZ(i), false);
-            const bool fluid_before = !solid_at(p, s, px + CX(i), py + CY(i), pz + CZ(i), true);
-            if (!(fluid_now && fluid_before)) continue;
-            const int qxl = (int)lx + CX(i), qyl = (int)ly + CY(i), qzl = (int)lz + CZ(i);
-            if (!(qxl >= 0 && qyl >= 0 && qzl >= 0 && qxl < (int)p.box_n[0] && qyl < (int)p.box_n[1] && qzl < (int)p.box_n[2])) continue;
-            const uint32_t k2 = ((uint32_t)qzl * p.box_n[1] + (uint32_t)qyl) * p.box_n[0] + (uint32_t)qxl;
-            rs += Rec<R>::macro(p, k2, 0);
-            cnt += (R)1;
-            R fp[19];
-            fp[0] = 0;
-            for (int j = 1; j < 19; j++) fp[j] = Rec<R>::fpost(p, k2, j);
-            const Moments<R> m2 = moments<R>(fp);
-            const R r2 = Rec<R>::macro(p, k2, 0);
-            const R u2[3] = {Rec<R>::macro(p, k2, 1), Rec<R>::macro(p, k2, 2), Rec<R>::macro(p, k2, 3)};
-            pis[3] += m2.sxy - r2 * u2[0] * u2[1];
-            pis[4] += m2.sxz - r2 * u2[0] * u2[2];
-            pis[5] += m2.syz - r2 * u2[1] * u2[2];
-            const R tr = (m2.sxx + m2.syy + m2.szz) / (R)3;
-            const R uu = u2[0] * u2[0] + u2[1] * u2[1] + u2[2] * u2[2];
-            pis[0] += m2.sxx - tr - r2 * (u2[0] * u2[0] - uu / (R)3);
-            pis[1] += m2.syy - tr - r2 * (u2[1] * u2[1] - uu / (R)3);
-            pis[2] += m2.szz - tr - r2 * (u2[2] * u2[2] - uu / (R)3);
-        }
+        // fluid neighbours plus their mean non-equilibrium stress (gathered
+        // above); the part gives up the refill's momentum
         const R rho = cnt > (R)0 ? rs / cnt : (R)1;
         R om[3];
         if (sizeof(R) == 8) { om[0] = (R)s.omega_d[0]; om[1] = (R)s.omega_d[1]; om[2] = (R)s.omega_d[2]; }
