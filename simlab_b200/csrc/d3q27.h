@@ -56,6 +56,9 @@ struct LevelParams {
     lbm::FastDiv div_nx, div_nxy;
     int per[3];
     int n_sponge, forcing, abs_u, total_p;
+    // something may read whole states in the outermost layer (a spinning part's
+    // box next to it): face and ghost cells are then written in all directions
+    int outer_read;
     // refinement: this level's exports and the neighbouring levels' buffers
     int has_child, has_parent;
     int ch_lo[3];

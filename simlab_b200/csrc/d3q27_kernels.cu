@@ -74,6 +74,35 @@ __device__ __forceinline__ void put(const LevelParams &p, uint32_t set, uint32_t
     for (int i = 0; i < 27; i++) s[(uint64_t)i * p.NP + n] = Pop<S>::enc(f[i], rng);
 }
 
+// the same, only the directions need(i) asks for: of a face, ghost or
+// restricted cell those that stream into a cell that is updated are read by
+// anyone (9 of 27 on a plane), and along x each store of a plane is a sector of
+// its own.  The random sequence steps as for all 27.
+template <class S, class Need>
+__device__ __forceinline__ void put_some(const LevelParams &p, uint32_t set, uint32_t n, const typename Pop<S>::real *f, Rng &rng, Need &&need) {
+    S *s = set_ptr_w<S>(p, set);
+#pragma unroll
+    for (int i = 0; i < 27; i++) {
+        const S v = Pop<S>::enc(f[i], rng);
+        if (need(i)) s[(uint64_t)i * p.NP + n] = v;
+    }
+}
+// does direction i lead from (x, y, z) to a cell off the lattice's outermost
+// layer (on a periodic axis every cell is)
+__device__ __forceinline__ bool leads_inside(const LevelParams &p, uint32_t x, uint32_t y, uint32_t z, int i) {
+    const uint32_t tx = x + CX(i) - 1u, ty = y + CY(i) - 1u, tz = z + CZ(i) - 1u;
+    return (p.per[0] || tx < p.NX - 2u) && (p.per[1] || ty < p.NY - 2u) && (p.per[2] || tz < p.NZ - 2u);
+}
+// the 11 values of a moment node (12 apart)
+__device__ __forceinline__ void load_node(const float *m, float *v) {
+    const float4 a = reinterpret_cast<const float4 *>(m)[0], b = reinterpret_cast<const float4 *>(m)[1], c = reinterpret_cast<const float4 *>(m)[2];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w; v[8] = c.x; v[9] = c.y; v[10] = c.z;
+}
+__device__ __forceinline__ void load_node(const double *m, double *v) {
+#pragma unroll
+    for (int j = 0; j < 11; j++) v[j] = m[j];
+}
+
 template <class R>
 struct Mom {
     R rho1, j[3], s[6];
@@ -611,6 +640,7 @@ __global__ void __launch_bounds__(BLK) k27_face(const __grid_constant__ LevelPar
     const uint32_t b = p.faces[kk];
     uint32_t x, y, z;
     coords(p, b, x, y, z);
+    const uint32_t bx = x, by = y, bz = z;
     if (!p.per[0]) x = min(max(x, 1u), p.NX - 2);
     if (!p.per[1]) y = min(max(y, 1u), p.NY - 2);
     if (!p.per[2]) z = min(max(z, 1u), p.NZ - 2);
@@ -641,7 +671,7 @@ __global__ void __launch_bounds__(BLK) k27_face(const __grid_constant__ LevelPar
     R f[27];
     rebuild<R>(rho, u, pp, f);
     Rng rng = cell_rng<S>(b, a.seed_mix);
-    put<S>(p, a.src, b, f, rng);
+    put_some<S>(p, a.src, b, f, rng, [&](int i) { return p.outer_read || leads_inside(p, bx, by, bz, i); });
 }
 
 // mshader.rs:742-775: fine ghosts from the parent's surface moments, linear in
@@ -670,8 +700,9 @@ __global__ void __launch_bounds__(BLK) k27_ghost(const __grid_constant__ LevelPa
         if ((o[0] & ~odd[0]) | (o[1] & ~odd[1]) | (o[2] & ~odd[2])) continue;
         const R w = (odd[0] ? (R)0.5 : (R)1) * (odd[1] ? (R)0.5 : (R)1) * (odd[2] ? (R)0.5 : (R)1);
         const uint64_t nd = ((uint64_t)(h0[2] + o[2]) * p.pn[1] + (h0[1] + o[1])) * p.pn[0] + (h0[0] + o[0]);
-        const R *ma = mp + (a.mold * pnodes + nd) * MW;
-        const R *mb = mp + (a.mnew * pnodes + nd) * MW;
+        R ma[11], mb[11];
+        load_node(mp + (a.mold * pnodes + nd) * MW, ma);
+        load_node(mp + (a.mnew * pnodes + nd) * MW, mb);
 #pragma unroll
         for (int j = 0; j < 11; j++) acc[j] += w * (((R)1 - blend) * ma[j] + blend * mb[j]);
         wsum += w;
@@ -687,7 +718,7 @@ __global__ void __launch_bounds__(BLK) k27_ghost(const __grid_constant__ LevelPa
     R f[27];
     rebuild<R>(rho, u, pp, f);
     Rng rng = cell_rng<S>(n, a.seed_mix);
-    put<S>(p, a.src, n, f, rng);
+    put_some<S>(p, a.src, n, f, rng, [&](int i) { return p.outer_read || leads_inside(p, xyz[0], xyz[1], xyz[2], i); });
 }
 
 // mshader.rs:777-793: coarse cells under the child box from its coincident nodes
@@ -701,7 +732,8 @@ __global__ void __launch_bounds__(BLK) k27_restrict(const __grid_constant__ Leve
     uint32_t x, y, z;
     coords(p, n, x, y, z);
     const uint32_t lx = x - (uint32_t)p.ch_lo[0], ly = y - (uint32_t)p.ch_lo[1], lz = z - (uint32_t)p.ch_lo[2];
-    const R *m = (const R *)p.mom_child_up + (((uint64_t)lz * p.ch_n[1] + ly) * p.ch_n[0] + lx) * MW;
+    R m[11];
+    load_node((const R *)p.mom_child_up + (((uint64_t)lz * p.ch_n[1] + ly) * p.ch_n[0] + lx) * MW, m);
     const R rho = m[0];
     const R u[3] = {m[1], m[2], m[3]};
     const R tf = m[10];
@@ -713,7 +745,11 @@ __global__ void __launch_bounds__(BLK) k27_restrict(const __grid_constant__ Leve
     R f[27];
     rebuild<R>(rho, u, pp, f);
     Rng rng = cell_rng<S>(n, a.seed_mix);
-    put<S>(p, a.src, n, f, rng);
+    // into the cells that are not restricted: off the box two nodes inside the child's
+    put_some<S>(p, a.src, n, f, rng, [&](int i) {
+        const uint32_t tx = lx + CX(i) - 2u, ty = ly + CY(i) - 2u, tz = lz + CZ(i) - 2u;
+        return tx > p.ch_n[0] - 5u || ty > p.ch_n[1] - 5u || tz > p.ch_n[2] - 5u;
+    });
 }
 
 // mshader.rs:520-527: feq(1, u_init) in both sets

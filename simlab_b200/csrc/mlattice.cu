@@ -585,6 +585,8 @@ void create_multi(const lbm_multi_setup *setup, const lbm_geometry *geom, const 
     if (spin) {
         lbm27::LevelParams &p = h->lv[finest].p;
         p.moving = 1;
+        for (int k = 0; k < 3; k++)
+            if (spin->box_lo[k] < 2 || (int64_t)spin->box_lo[k] + (int64_t)spin->box_n[k] > (int64_t)fd[k] - 2) p.outer_read = 1;
         const uint64_t nocc = (uint64_t)spin->occ_dims[0] * spin->occ_dims[1] * spin->occ_dims[2];
         const uint64_t wocc = (nocc + 31) / 32;
         p.occ = (const uint32_t *)h->dalloc(wocc * 4);
