@@ -270,7 +270,7 @@ __device__ __forceinline__ void relax(const LatParams &p, const Consts<R> &k, R 
 template <class S, int P, int COLL>
 __global__ void __launch_bounds__(BLOCK) k_bulk(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
     using R = typename Pop<S>::real;
-    const uint32_t n = blockIdx.x * BLOCK + threadIdx.x;
+    const uint32_t n = (P == 1 ? gridDim.x - 1u - blockIdx.x : blockIdx.x) * BLOCK + threadIdx.x;  // (tile_start's order)
     if (n >= p.N) return;
     if ((p.flags[n] & ~FLAG_XFACE) != 0u) return;
     uint32_t x, y, z;
@@ -647,6 +647,16 @@ __device__ __forceinline__ int64_t plane_shift(int j, int64_t NX, int64_t NXY) {
     return (P == 0 || j == 0) ? 0 : (int64_t)CX(j) + (int64_t)CY(j) * NX + (int64_t)CZ(j) * NXY;
 }
 
+// First cell of the t-th tile a step takes.  The lattice is updated in place
+// and the parities alternate, so one parity walks it backwards: a step starts on
+// the cells the step before wrote last, which L2 (126 MB) still holds.  ms per
+// batch, forwards -> in turn: FP32 203x131x117 (249 MB) 23.5 -> 22.5, the direct
+// kernel's 131x130x129 FP32 27.6 -> 25.7, FP16 512x256x256 (1.3 GB) 11.53 -> 11.45.
+template <int P>
+__device__ __forceinline__ uint32_t tile_start(uint32_t t, uint32_t ntiles, uint32_t T) {
+    return (P == 1 ? ntiles - 1u - t : t) * T;
+}
+
 // The loads of tile n0 into a buffer by producer warp pw of NPROD: the
 // planes j = pw (mod NPROD), and the flags from the last producer; each
 // producer posts its own bytes on the buffer's "full" barrier.
@@ -957,7 +967,7 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
                     // and slots clamped to [0, N); the 16-byte-aligned interior
                     // with one bulk store, the ragged ends with plain stores
                     const int j = pw + NPROD * lane;
-                    const uint32_t n0 = (blockIdx.x + (it - NBUF) * G) * T;
+                    const uint32_t n0 = tile_start<P>(blockIdx.x + (it - NBUF) * G, ntiles, T);
                     const int64_t sh = tab_sh[j];
                     const int64_t lo = max((int64_t)n0, -sh);
                     int64_t hi = min(min((int64_t)n0 + (int64_t)T, N), N - sh);
@@ -981,7 +991,7 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
             if (it + 1 == K) pdl_release();
             if (it < K && lane == 0) {
                 fence_async_smem();
-                tma_load_tile<S, P, NPROD, RAG>(p, sm + b * BUF, &full[b], (blockIdx.x + it * G) * T, pw);
+                tma_load_tile<S, P, NPROD, RAG>(p, sm + b * BUF, &full[b], tile_start<P>(blockIdx.x + it * G, ntiles, T), pw);
             }
         }
         if (!alive && lane == 0) {
@@ -1009,7 +1019,7 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
         }
         uint8_t *buf = sm + b * BUF;
         const uint32_t *fl = (const uint32_t *)(buf + 19 * SLOT);
-        const uint32_t n0 = t * T;
+        const uint32_t n0 = tile_start<P>(t, ntiles, T);
         if constexpr (sizeof(S) == 2 && COLL == 0 && FEAT != 0) {
             bulk_pairs<S, P, FEAT, RAG>(p, s, buf, n0, zper);
         } else
