@@ -8,8 +8,9 @@
 //   k_walls  -- wall-record cells: streaming + Bouzidi / moving-wall links +
 //               collision (shader.rs:795-862 with $WALLS$ 399-436), and the
 //               momentum-exchange force and moment summed in FP64 with warp
-//               shuffles, per block, then by the last block in a fixed order
-//               (replaces reduce1/reduce2, shader.rs:689-734).
+//               shuffles, per block; k_force_sum adds the blocks of a batch's
+//               steps in a fixed order (replaces reduce1/reduce2,
+//               shader.rs:689-734).
 //   k_bulk   -- every other fluid cell: fused AA stream + collide.
 // k_walls and k_bulk touch disjoint cells; in the AA pattern every memory
 // slot is read and written by exactly one thread per step, so they need no
@@ -1439,15 +1440,6 @@ static void launch_tma(const LatParams &p, const StepParams &s, cudaStream_t st,
         }
     }
     launch_pdl(pdl, k_bulk_tma<S, P, COLL, FEAT, false>, std::min(ntiles, tma_grid<S, P, COLL, FEAT, false>()), Tma<S>::threads, tma_smem<S>(), st, p, s);
-}
-
-uint32_t staged_tile_cells(int storage) {
-    switch (storage) {
-        case 0: return Tile<float>::cells;
-        case 1: return Tile<__half>::cells;
-        case 2: return Tile<__nv_bfloat16>::cells;
-        default: return Tile<double>::cells;
-    }
 }
 
 // One step: faces and wall cells, then the bulk.  Where no wall cell is near a

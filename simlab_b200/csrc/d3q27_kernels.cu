@@ -910,7 +910,7 @@ __global__ void __launch_bounds__(BLK) k27_tri_scatter(const __grid_constant__ L
     lbm::pdl_wait();
     // one warp per triangle, its lanes over the lattice points near it
     // (the blocks past the triangles' classify the box's cells)
-    const uint32_t tri_blocks = (p.ntri * 32u + BLK - 1) / BLK;
+    const uint32_t tri_blocks = (uint32_t)(((uint64_t)p.ntri * 32u + BLK - 1) / BLK);
     if (blockIdx.x >= tri_blocks) {
         sp27::solid_cell(p, a, (blockIdx.x - tri_blocks) * BLK + threadIdx.x);
         return;

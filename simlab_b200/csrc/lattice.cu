@@ -403,10 +403,11 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
     const bool tma_ok = !per[0] && !per[1] && !(no_tma && no_tma[0] == '1') &&
                         (!ragged || st.storage == LBM_STORAGE_FP64 ||
                          (N >= ragged_from && st.collision == LBM_COLLISION_REGULARIZED && !force && !st.absorb_velocity && !per[2]));
-    const uint64_t tile = lbm::staged_tile_cells(st.storage);
     std::vector<char> fused(faces.size(), 0);
     uint32_t xinfo[2] = {0, 0};
-    // (not with a spinning part, whose re-voxelizer rewrites the box flags)
+    // (not with a spinning part, whose re-voxelizer rewrites the box flags, and
+    // not on ragged rows, where a pair may lie in two tiles and the face
+    // kernel's roundings are the ones to keep)
     if (tma_ok && !spin && !ragged) {
         for (size_t k = 0; k < faces.size(); k++) {
             const uint64_t c = faces[k], x = c % NX, y = (c / NX) % NY, z = c / (NX * NY);
@@ -416,8 +417,6 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
             if (y == 0 || y == NY - 1 || z == 0 || z == NZ - 1) continue;
             const uint64_t m = x == 0 ? c + 1 : c - 1;
             if (flags[m] != 0) continue;
-            // both in one staged tile (rows of odd length put some pairs across two)
-            if (c / tile != m / tile) continue;
             fused[k] = 1;
             flags[m] |= lbm::FLAG_XFACE;
             xinfo[x == 0 ? 0 : 1] = finfo[k] & 0xffu;
@@ -586,12 +585,11 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
         p.ntri = (uint32_t)spin->ntri;
         p.tris = (const float4 *)h->dalloc(std::max<uint64_t>(spin->ntri, 1) * 48);
         if (spin->ntri) ck(cudaMemcpy((void *)p.tris, spin->tris, spin->ntri * 48, cudaMemcpyHostToDevice), "upload triangles");
-        std::vector<uint32_t> q0((size_t)nrec * 54, 0u);
-        for (size_t w = 0; w < 54; w += 3)
-            std::fill_n(q0.begin() + (ptrdiff_t)(w * nrec), nrec, 0x7f7fffffu);  // nearest hit: FLT_MAX
-        p.qscr = (uint32_t *)h->dalloc(q0.size() * 4);
+        // link scratch: hits 0, farthest 0, nearest beyond any (0x7f7f7f7f)
+        p.qscr = (uint32_t *)h->dalloc((uint64_t)nrec * 54 * 4);
+        ck(cudaMemsetAsync(p.qscr, 0, (uint64_t)nrec * 54 * 4, h->stream), "memset");
+        for (uint64_t w = 0; w < 54; w += 3) ck(cudaMemsetAsync(p.qscr + w * nrec, 0x7f, nrec * 4, h->stream), "memset");
         p.sol = (uint8_t *)h->dalloc(((uint64_t)spin->box_n[0] + 2) * (spin->box_n[1] + 2) * (spin->box_n[2] + 2));
-        ck(cudaMemcpy(p.qscr, q0.data(), q0.size() * 4, cudaMemcpyHostToDevice), "upload link scratch");
     }
     fill_consts<float>(p.kf, st);
     fill_consts<double>(p.kd, st);

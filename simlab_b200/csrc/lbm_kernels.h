@@ -22,8 +22,6 @@ cudaError_t launch_step(int storage, const LatParams &p, const StepParams &s, in
 // force and moment of the steps whose partials are kept, into the history
 // slots slot0, slot0 + 1, ...
 cudaError_t launch_force_sum(const LatParams &p, uint32_t slot0, uint32_t steps, cudaStream_t st);
-// cells of one tile of the staged bulk kernel: tiles start at its multiples
-uint32_t staged_tile_cells(int storage);
 cudaError_t launch_init(int storage, const LatParams &p, cudaStream_t st);
 cudaError_t launch_dump(int storage, const LatParams &p, int q, cudaStream_t st);
 cudaError_t launch_sample(int storage, const LatParams &p, const StepParams &s, int q, const float *verts, uint32_t nvert, float voff,

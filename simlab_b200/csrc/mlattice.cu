@@ -601,12 +601,11 @@ void create_multi(const lbm_multi_setup *setup, const lbm_geometry *geom, const 
         p.ntri = (uint32_t)spin->ntri;
         p.tris = (const float4 *)h->dalloc(std::max<uint64_t>(spin->ntri, 1) * 48);
         if (spin->ntri) ck(cudaMemcpy((void *)p.tris, spin->tris, spin->ntri * 48, cudaMemcpyHostToDevice), "upload triangles");
-        std::vector<uint32_t> q0((size_t)h->nrec * 78, 0u);
-        for (size_t w = 0; w < 78; w += 3)
-            std::fill_n(q0.begin() + (ptrdiff_t)(w * h->nrec), h->nrec, 0x7f7fffffu);  // nearest hit: FLT_MAX
-        p.qscr = (uint32_t *)h->dalloc(q0.size() * 4);
+        // link scratch: hits 0, farthest 0, nearest beyond any (0x7f7f7f7f)
+        p.qscr = (uint32_t *)h->dalloc((uint64_t)h->nrec * 78 * 4);
+        ck(cudaMemsetAsync(p.qscr, 0, (uint64_t)h->nrec * 78 * 4, h->stream), "memset");
+        for (uint64_t w = 0; w < 78; w += 3) ck(cudaMemsetAsync(p.qscr + w * h->nrec, 0x7f, (uint64_t)h->nrec * 4, h->stream), "memset");
         p.sol = (uint8_t *)h->dalloc(((uint64_t)spin->box_n[0] + 2) * (spin->box_n[1] + 2) * (spin->box_n[2] + 2));
-        ck(cudaMemcpy(p.qscr, q0.data(), q0.size() * 4, cudaMemcpyHostToDevice), "upload link scratch");
     }
     for (size_t l = 0; l < nl; l++) {
         lbm27::LevelParams &p = h->lv[l].p;

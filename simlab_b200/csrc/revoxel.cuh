@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(BLOCK) k_tri_scatter(const __grid_constant__ L
     pdl_wait();
     // one warp per triangle, its lanes over the lattice points near it
     // (the blocks past the triangles' classify the box's cells)
-    const uint32_t tri_blocks = (p.ntri * 32u + BLOCK - 1) / BLOCK;
+    const uint32_t tri_blocks = (uint32_t)(((uint64_t)p.ntri * 32u + BLOCK - 1) / BLOCK);
     if (blockIdx.x >= tri_blocks) {
         solid_cell(p, s, (blockIdx.x - tri_blocks) * BLOCK + threadIdx.x);
         return;
