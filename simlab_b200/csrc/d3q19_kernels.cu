@@ -501,7 +501,6 @@ __device__ __forceinline__ void faces_cell(const LatParams &p, const StepParams 
 
 template <class S, int P>
 __global__ void __launch_bounds__(BLOCK) k_faces(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
-    pdl_release();
     // beside the wall kernel (no wall cell near a face, so neither touches what
     // the other does): the wall kernel let this one start after its own wait for
     // the step before, and one thread's wait at the end keeps this grid from
@@ -986,10 +985,6 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
                 }
                 __syncwarp();
             }
-            // the next kernel's blocks may come once every block is at its last
-            // tile: let in earlier, they all crowd onto the SMs whose blocks
-            // finish first (the 512x256x256 FP16 step 30 us longer)
-            if (it + 1 == K) pdl_release();
             if (it < K && lane == 0) {
                 fence_async_smem();
                 tma_load_tile<S, P, NPROD, RAG>(p, sm + b * BUF, &full[b], tile_start<P>(blockIdx.x + it * G, ntiles, T), pw);

@@ -3,12 +3,14 @@
 // completed, memory included (pdl_wait), and its blocks are launched as the
 // last blocks of that one exit instead of after a launch gap of 2-3 us.  Since
 // every kernel waits for its predecessor, a completed kernel implies all
-// earlier ones.  pdl_release lets the next grid in earlier; only the wall and
-// face kernels (whose successors run beside them or fill every SM evenly) and
-// the staged bulk's last tile use it: let in while a kernel runs, a small
-// grid's blocks crowd onto the SMs that have room first and run there several
-// at a time (the rotor's face kernel 66 us instead of 26).  Without the launch
-// attribute both instructions do nothing.
+// earlier ones.  pdl_release lets the next grid in earlier; only the wall
+// kernel uses it, for the face kernel that runs beside it.  Let in while a
+// kernel runs, a small grid's blocks crowd onto the SMs that have room first
+// and run there several at a time: the rotor's face kernel took 66 us instead
+// of 26, and letting the next grid in at the staged bulk's last tile cost 99 us
+// a step instead of 85 (256x128x128 FP16, a part at rest; at the bulk's start
+// 30 us more on 512x256x256).  Without the launch attribute both instructions
+// do nothing.
 #pragma once
 #include <cuda_runtime.h>
 
