@@ -210,7 +210,9 @@ int lbm_synchronize(lbm_lattice *h);
 /* Per-kernel device time of the steps enqueued while profiling is on,
  * from CUDA events recorded around each kernel on the handle's stream (no
  * reference counterpart; for the roofline figures), and the number of
- * kernels those steps launched.  Enabling clears the totals;
+ * kernels those steps launch when they are not timed one by one (with
+ * enable 1 the wall and face cells, which otherwise share a grid where no
+ * wall cell is near a face, take a kernel each).  Enabling clears the totals;
  * lbm_kernel_times waits for the stream and returns them. */
 typedef struct {
     uint64_t steps;

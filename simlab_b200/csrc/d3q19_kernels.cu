@@ -410,16 +410,17 @@ __device__ __forceinline__ void face_planar(const LatParams &p, const StepParams
     });
 }
 
+// thread t of the face list's block blk of BLOCK cells
 template <class S, int P>
-__device__ __forceinline__ void faces_cell(const LatParams &p, const StepParams &s) {
+__device__ __forceinline__ void faces_cell(const LatParams &p, const StepParams &s, uint32_t blk, uint32_t t) {
     using R = typename Pop<S>::real;
     constexpr int Q = 1 - P;
     // the block's group: planar cells of one face (F < 6), or the rest
     int F = 6;
 #pragma unroll
     for (int g = 5; g >= 0; g--)
-        if (blockIdx.x < p.fblk[g + 1]) F = g;
-    const uint32_t kf = p.fplan[F] + (blockIdx.x - p.fblk[F]) * BLOCK + threadIdx.x;
+        if (blk < p.fblk[g + 1]) F = g;
+    const uint32_t kf = p.fplan[F] + (blk - p.fblk[F]) * BLOCK + t;
     if (kf >= (F < 6 ? p.fplan[F + 1] : s.nface)) return;
     uint32_t b, info;
     if (F < 6 && p.frect[F]) {
@@ -501,13 +502,8 @@ __device__ __forceinline__ void faces_cell(const LatParams &p, const StepParams 
 
 template <class S, int P>
 __global__ void __launch_bounds__(BLOCK) k_faces(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
-    // beside the wall kernel (no wall cell near a face, so neither touches what
-    // the other does): the wall kernel let this one start after its own wait for
-    // the step before, and one thread's wait at the end keeps this grid from
-    // completing before the wall kernel has
-    if (!s.beside) pdl_wait();
-    faces_cell<S, P>(p, s);
-    if (s.beside && blockIdx.x == 0 && threadIdx.x == 0) pdl_wait();
+    pdl_wait();
+    faces_cell<S, P>(p, s, blockIdx.x, threadIdx.x);
 }
 
 // ---------------------------------------------------------------- staged bulk
@@ -1189,14 +1185,13 @@ __device__ __forceinline__ void record_after(const LatParams &p, uint32_t r, con
     }
 }
 
+// block blk of nblk of the wall records
 template <class S, int P, int COLL>
-__global__ void __launch_bounds__(WBLOCK) k_walls(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
+__device__ __forceinline__ void walls_block(const LatParams &p, const StepParams &s, uint32_t blk, uint32_t nblk) {
     using R = typename Pop<S>::real;
     const Consts<R> &k = K<R>(p);
-    const uint32_t r = blockIdx.x * WBLOCK + threadIdx.x;
+    const uint32_t r = blk * WBLOCK + threadIdx.x;
     R Fo[3] = {0, 0, 0}, To[3] = {0, 0, 0};
-    pdl_wait();
-    pdl_release();
     if (r < p.nrec) {
         // The record's first 32 words, the cell's flag and its 19 populations
         // issued together before anything waits on them: the wall kernel is
@@ -1229,7 +1224,35 @@ __global__ void __launch_bounds__(WBLOCK) k_walls(const __grid_constant__ LatPar
     }
     // FP64 sum: warp shuffle -> block partial (k_force_sum adds the blocks)
     double v[6] = {(double)Fo[0], (double)Fo[1], (double)Fo[2], (double)To[0], (double)To[1], (double)To[2]};
-    block_partial6<WBLOCK>(v, p.partials + ((uint64_t)s.part * gridDim.x + blockIdx.x) * 8);
+    block_partial6<WBLOCK>(v, p.partials + ((uint64_t)s.part * nblk + blk) * 8);
+}
+
+template <class S, int P, int COLL>
+__global__ void __launch_bounds__(WBLOCK) k_walls(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
+    pdl_wait();
+    walls_block<S, P, COLL>(p, s, blockIdx.x, gridDim.x);
+}
+
+// The wall cells and the face cells in one grid, where no wall cell is near a
+// face, so neither touches what the other does: the first blocks take the
+// records, the others the face list in blocks of WBLOCK.  Both jobs are short
+// and bound by latency; every thread waits for the step before ahead of its
+// first load.  Against the wall kernel and the face kernel beside it as two
+// grids, ms per batch: 96x48x48 FP32 (256 steps) 4.84 -> 4.65, 203x131x117 FP32
+// (224) 21.4 -> 21.3, 512x256x256 FP16 (20) 11.46 -> 11.37, 301x157x157 BF16 (94)
+// 13.6 -> 13.7.
+template <class S, int P, int COLL>
+__global__ void __launch_bounds__(WBLOCK) k_walls_faces(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
+    static_assert(BLOCK % WBLOCK == 0, "the face list's blocks are split evenly");
+    constexpr uint32_t SUB = BLOCK / WBLOCK;
+    pdl_wait();
+    const uint32_t nw = (p.nrec + WBLOCK - 1) / WBLOCK;
+    if (blockIdx.x < nw) {
+        walls_block<S, P, COLL>(p, s, blockIdx.x, nw);
+    } else {
+        const uint32_t q = blockIdx.x - nw;
+        faces_cell<S, P>(p, s, q / SUB, q % SUB * WBLOCK + threadIdx.x);
+    }
 }
 
 // ---------------------------------------------------------------- init
@@ -1438,26 +1461,18 @@ static void launch_tma(const LatParams &p, const StepParams &s, cudaStream_t st,
 }
 
 // One step: faces and wall cells, then the bulk.  Where no wall cell is near a
-// face (walls_far) the wall kernel goes first and the face kernel runs beside
-// it; in a periodic box, which has no faces, the direct bulk kernel does, from
-// the stream `side` (131x130x129 FP32: the wall kernel's 15 us beside the bulk's
-// 69 instead of before them).  The direct kernel is launched as any other, not
-// with programmatic serialization: a wait in it changes which of its products
-// the compiler fuses.  ev:
-// null, or events to record (null entries are left out); with events between
-// the kernels these run one by one.
+// face (walls_with_faces) one grid takes both; in a periodic box, which has no
+// faces, the wall kernel runs beside the direct bulk kernel, from the stream
+// `side` (131x130x129 FP32: the wall kernel's 15 us beside the bulk's 69 instead
+// of before them).  The direct kernel is launched as any other, not with
+// programmatic serialization: a wait in it changes which of its products the
+// compiler fuses.  ev: null, or events to record (null entries are left out);
+// with events between the kernels these run one by one.
 template <class S, int P, int COLL>
-static cudaError_t step_t(const LatParams &p, const StepParams &s0, cudaStream_t st, const WallsBeside &wb, cudaEvent_t *ev) {
+static cudaError_t step_t(const LatParams &p, const StepParams &s, cudaStream_t st, const WallsBeside &wb, cudaEvent_t *ev) {
     const bool pdl = !(ev && ev[0]);
-    StepParams s = s0;
-    s.beside = 0;
     const unsigned wgrid = (unsigned)((p.nrec + WBLOCK - 1) / WBLOCK);
-    auto walls = [&] { launch_pdl(pdl, k_walls<S, P, COLL>, wgrid, WBLOCK, 0, st, p, s); };
-    auto faces = [&](int beside) {
-        s.beside = beside;
-        launch_pdl(pdl, k_faces<S, P>, p.fblk[6] + blocks_for(s.nface - p.fplan[6]), BLOCK, 0, st, p, s);
-        s.beside = 0;
-    };
+    const unsigned fgrid = p.fblk[6] + blocks_for(s.nface - p.fplan[6]);
     if (ev && ev[0]) cudaEventRecord(ev[0], st);
     if (p.moving) {
         // re-voxelize the spinning part's swept box for this step's rotation
@@ -1466,18 +1481,18 @@ static cudaError_t step_t(const LatParams &p, const StepParams &s0, cudaStream_t
         launch_pdl(pdl, k_tri_scatter, blocks_for((uint64_t)p.ntri * 32u) + blocks_for(halo), BLOCK, 0, st, p, s);
         launch_pdl(pdl, k_voxelize<S, 1 - P>, blocks_for(p.nrec), BLOCK, 0, st, p, s);
     }
-    const bool overlap = pdl && wb.far && p.nrec && s.nface && !p.moving;
+    const bool shared = pdl && walls_with_faces(p, s, wb);
     const bool aside = pdl && wb.side && p.nrec && !p.moving;
-    if (overlap) walls();
-    if (s.nface) faces(overlap ? 1 : 0);
+    if (shared) launch_pdl(pdl, k_walls_faces<S, P, COLL>, wgrid + fgrid * (BLOCK / WBLOCK), WBLOCK, 0, st, p, s);
+    else if (s.nface) launch_pdl(pdl, k_faces<S, P>, fgrid, BLOCK, 0, st, p, s);
     if (ev && ev[1]) cudaEventRecord(ev[1], st);
     if (aside) {
         cudaEventRecord(wb.fork, st);
         cudaStreamWaitEvent(wb.side, wb.fork, 0);
         k_walls<S, P, COLL><<<wgrid, WBLOCK, 0, wb.side>>>(p, s);
         cudaEventRecord(wb.join, wb.side);
-    } else if (p.nrec && !overlap) {
-        walls();
+    } else if (p.nrec && !shared) {
+        launch_pdl(pdl, k_walls<S, P, COLL>, wgrid, WBLOCK, 0, st, p, s);
     }
     if (ev && ev[2]) cudaEventRecord(ev[2], st);
     if (p.tma) {

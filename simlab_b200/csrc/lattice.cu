@@ -623,8 +623,8 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
     }
     p.sp_tab = (const float *)h->dalloc(tabf.size() * 4);
     p.sp_tabd = (const double *)h->dalloc(tabd.size() * 8);
-    // the wall kernel may overlap the face kernel when no wall cell is within
-    // three cells of a non-periodic boundary (its slots then never meet the
+    // wall and face cells may share a grid when no wall cell is within three
+    // cells of a non-periodic boundary (a wall cell's slots then never meet the
     // faces' slots or the inner cells the faces read)
     bool walls_far = nrec > 0 && !faces.empty() && !spin;
     for (uint64_t r = 0; walls_far && r < nrec; r++) {
@@ -690,8 +690,8 @@ void run_impl(lbm_lattice *h, const lbm_step_in *steps, uint64_t n, double *forc
                     evs = ev4;
                 }
                 h->prof_steps++;
-                // the kernels launch_step enqueues for this step
-                h->prof_launches += (sp.nface ? 1u : 0u) + (p.nrec ? 1u : 0u) + 1u + (p.moving ? 2u : 0u);
+                // the kernels launch_step enqueues for this step when it is not split for timing
+                h->prof_launches += (sp.nface ? 1u : 0u) + (p.nrec ? 1u : 0u) + 1u + (p.moving ? 2u : 0u) - (lbm::walls_with_faces(p, sp, h->walls_beside) ? 1u : 0u);
                 if (si.sample) h->prof_launches += (h->nvert ? 1u : 0u) + (h->npix ? 1u : 0u);
             }
             ck(lbm::launch_step(h->setup.storage, p, sp, (int)(idx % 2), h->setup.collision, h->stream, h->walls_beside, evs),

@@ -174,7 +174,6 @@ struct StepParams {
     uint32_t nface;          // face cells the face kernel handles this step
     uint32_t part;   // the step's place among the kept block partials
     uint32_t scr;    // link scratch set of this step
-    int beside;      // this kernel runs beside the wall kernel, not after it
     float omega[3];  // angular velocity, rad per step
     double omega_d[3];
     float rot[9];    // body axes in lattice coordinates, row-major (columns = axes)

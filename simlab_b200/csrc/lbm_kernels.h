@@ -7,14 +7,17 @@
 namespace lbm {
 
 // storage: 0 FP32, 1 FP16, 2 BF16, 3 FP64 (lbm_storage); coll: 0 regularized, 1 BGK
-// What the wall kernel may run beside: the face kernel (far: no wall cell is
-// near a face), or the direct bulk kernel of a lattice without faces, from a
-// second stream (side, with the two events that fork it off and join it).
+// What the wall cells may be updated beside: the face cells, in one grid (far:
+// no wall cell is near a face), or the direct bulk kernel of a lattice without
+// faces, from a second stream (side, with the two events that fork it off and
+// join it).
 struct WallsBeside {
     bool far = false;
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
 };
+// whether one grid takes the step's wall and face cells
+inline bool walls_with_faces(const LatParams &p, const StepParams &s, const WallsBeside &wb) { return wb.far && p.nrec && s.nface && !p.moving; }
 // ev: null, or 4 events recorded before the step, after faces,
 // after walls, after bulk
 cudaError_t launch_step(int storage, const LatParams &p, const StepParams &s, int parity, int coll, cudaStream_t st, const WallsBeside &wb,
