@@ -392,17 +392,18 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
     const bool force = st.body_force[0] != 0.0 || st.body_force[1] != 0.0 || st.body_force[2] != 0.0;
     // Rows that are no whole number of 16-byte units take the staged kernel's
     // ragged variant where it rounds as the direct kernel does: the
-    // regularized collision without a body force, without the u_inf absorbing
-    // target and without periodic z (and FP64, whose roundings no result shows).
-    // Small lattices stay with it too: the staged kernel's few large tiles leave
-    // SMs idle.  Measured, us per step of a sphere in a tunnel, direct / staged:
-    // FP32 0.41 M cells 26.7 / 28.7, 0.82 M 36.0 / 36.8, 1.7 M 73.4 / 70.5, 3.6 M
-    // 134.6 / 122.3; FP16 28.2 / 31.3, 41.1 / 37.8, 67.0 / 52.0, 134.6 / 90.1
-    // (BF16 like FP16); FP64 27.6 / 27.6 at 0.1 M, 231 / 230 at 3.6 M.
+    // regularized collision in FP32 without a body force, without the u_inf
+    // absorbing target and without periodic z.  Small lattices stay with the
+    // direct kernel too: the staged kernel's few large tiles leave SMs idle.
+    // Measured, us per step of a sphere in a tunnel, direct / staged: FP32 0.41 M
+    // cells 26.7 / 28.7, 0.82 M 36.0 / 36.8, 1.7 M 73.4 / 70.5, 3.6 M 134.6 /
+    // 122.3; FP16 28.2 / 31.3, 41.1 / 37.8, 67.0 / 52.0, 134.6 / 90.1 (BF16 like
+    // FP16).  FP64 stays with it at every size: 27.6 / 27.6 at 0.1 M, 231 / 230 at
+    // 3.6 M, for other roundings.
     const uint64_t ragged_from = st.storage == LBM_STORAGE_FP32 ? 1000000 : 640000;
     const bool tma_ok = !per[0] && !per[1] && !(no_tma && no_tma[0] == '1') &&
-                        (!ragged || st.storage == LBM_STORAGE_FP64 ||
-                         (N >= ragged_from && st.collision == LBM_COLLISION_REGULARIZED && !force && !st.absorb_velocity && !per[2]));
+                        (!ragged || (st.storage != LBM_STORAGE_FP64 && N >= ragged_from && st.collision == LBM_COLLISION_REGULARIZED &&
+                                     !force && !st.absorb_velocity && !per[2]));
     std::vector<char> fused(faces.size(), 0);
     uint32_t xinfo[2] = {0, 0};
     // (not with a spinning part, whose re-voxelizer rewrites the box flags, and
