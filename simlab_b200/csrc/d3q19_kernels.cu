@@ -526,9 +526,9 @@ __global__ void __launch_bounds__(BLOCK) k_faces(const __grid_constant__ LatPara
 // lengths (RAG) the misalignment is still one number per plane, since tiles
 // start at whole units: it comes with the parameters, at one more addition per
 // access.  203 x 131 x 117 FP32: bulk 92 us per step with the direct kernel
-// (average of the parities), 80 staged; 301 x 157 x 157 BF16: 227 and 120.  Store ranges
-// are clamped to real cells and real slots, so no two blocks write the same
-// slot.  Requires non-periodic x and y; a periodic z wraps only at the z
+// (average of the parities), 80 staged; 301 x 157 x 157 BF16: 227 and 120.
+// Store ranges are clamped to real cells and real slots, so no two blocks write
+// the same slot.  Requires non-periodic x and y; a periodic z wraps only at the z
 // boundaries, where cells load and store their wrapped links directly.
 //
 // Blocks are persistent and double buffered (the next tile's copies are in
@@ -552,10 +552,10 @@ __global__ void __launch_bounds__(BLOCK) k_faces(const __grid_constant__ LatPara
 // 2, 3, 4, 5 producer warps 59.8, 60.3, 60.5, 58.7 k FP16 (FP32 38.2 k with 2 or
 // 3).  With two cells per thread (bulk_pairs), us per FP16 step: 20 warps and
 // 2560 cells 493, 16 and 2048 537, 14 and 2688 525, 12 and 2304 557, 10 and
-// 2560 572, so the shape stays.  The copy engine takes a few hundred cycles per bulk copy (one per plane
-// and tile, each way) and the copies one warp issues go one after another, so
-// fewer, larger copies and several issuing warps shorten a buffer's
-// turnaround.
+// 2560 572, so the shape stays.  The copy engine takes a few hundred cycles per
+// bulk copy (one per plane and tile, each way) and the copies one warp issues go
+// one after another, so fewer, larger copies and several issuing warps shorten a
+// buffer's turnaround.
 #ifndef LBM_CWARPS_2B
 #define LBM_CWARPS_2B 20  // compute warps per block for 2-byte storage
 #endif
@@ -673,19 +673,13 @@ __device__ __forceinline__ void tma_load_tile(const LatParams &p, uint8_t *buf, 
     if (pw == NPROD - 1) bulk_g2s(buf + 19 * SLOT, p.flags + n0, T * 4, bar);
 }
 
-// The x-face cell b next to cell m (b = m - 1 when x = 1, b = m + 1 when
-// x = NX - 2), on a planar x face whose inner neighbour is m: its populations
-// for the next step are what the face kernel of the next step would write
-// from m's post-collision state, so the thread that just collided m computes
-// them from its rounded outputs and writes them into b's slots of the staged
-// tile; they reach HBM with the tile.  Only the 5 directions entering the
-// domain are needed (the face kernel's store mask for a planar x face).
+// the 5 directions entering the domain at a planar x face
 __host__ __device__ __forceinline__ constexpr int inward_dir(bool lo, int q) {
     // c_x = +1 directions (face at x = 0) or c_x = -1 (face at x = NX - 1), ascending
     return lo ? (q == 0 ? 1 : (q == 1 ? 7 : (q == 2 ? 9 : (q == 3 ? 13 : 15)))) : (q == 0 ? 2 : (q == 1 ? 8 : (q == 2 ? 10 : (q == 3 ? 14 : 16))));
 }
 
-template <class S, int P, bool LO, bool RAG>
+template <class S, int P, bool LO>
 __device__ __forceinline__ void xface_side(const LatParams &p, const StepParams &s, uint8_t *buf, uint32_t c, uint32_t m, uint32_t y,
                                            uint32_t z, const S *out) {
     using R = typename Pop<S>::real;
@@ -738,7 +732,7 @@ __device__ __forceinline__ void xface_side(const LatParams &p, const StepParams 
         if (!p.per[2] && (tz <= 0 || tz >= (int64_t)p.NZ - 1)) continue;
         const S v = Pop<S>::enc(fb[q], rng);
         const int j = P == 0 ? OPP(i) : i;
-        ((S *)(buf + j * SLOT))[lead_of<S, P, RAG>(p, j) + cb] = v;
+        ((S *)(buf + j * SLOT))[lead<S, P>(j) + cb] = v;
     }
 }
 
@@ -749,18 +743,20 @@ __device__ __forceinline__ void xface_side(const LatParams &p, const StepParams 
 // collided m computes them from its rounded outputs, with the face kernel's
 // arithmetic and random sequence, and writes them into b's slots of the
 // staged tile; they reach HBM with the tile.  Only the 5 directions entering
-// the domain are needed (the face kernel's store mask of a planar x face).
-template <class S, int P, bool RAG>
+// domain are needed (the face kernel's store mask of a planar x face).  Not on
+// ragged rows, where b may lie in another tile.
+template <class S, int P>
 __device__ __forceinline__ void xface_from_inner(const LatParams &p, const StepParams &s, uint8_t *buf, uint32_t c, uint32_t m, uint32_t x,
                                                  uint32_t y, uint32_t z, const S *out) {
-    if (x == 1) xface_side<S, P, true, RAG>(p, s, buf, c, m, y, z, out);
-    else xface_side<S, P, false, RAG>(p, s, buf, c, m, y, z, out);
+    if (x == 1) xface_side<S, P, true>(p, s, buf, c, m, y, z, out);
+    else xface_side<S, P, false>(p, s, buf, c, m, y, z, out);
 }
 
 // A cell of a periodic-z boundary plane at input parity 1: the links that
 // leave the domain in z wrap to the other side, so those inputs and outputs go
-// straight to HBM; the others use the staged tile like every other cell.
-template <class S, int COLL, bool RAG>
+// straight to HBM; the others use the staged tile like every other cell.  (No
+// periodic z on ragged rows.)
+template <class S, int COLL>
 __device__ __forceinline__ void zwrap_cell(const LatParams &p, const StepParams &s, uint8_t *buf, uint32_t c, uint32_t n, uint32_t x,
                                         uint32_t y, uint32_t z) {
     using R = typename Pop<S>::real;
@@ -773,7 +769,7 @@ __device__ __forceinline__ void zwrap_cell(const LatParams &p, const StepParams 
     for (int i = 0; i < 19; i++) {
         const int j = i == 0 ? 0 : OPP(i);
         if (i > 0 && CZ(i) == -zw) f[i] = Pop<S>::ld(pop + (uint64_t)j * p.NP + (uint32_t)((int32_t)n + nb.off(-CX(i), -CY(i), -CZ(i))));
-        else f[i] = Pop<S>::cvt(((const S *)(buf + j * SLOT))[lead_of<S, 1, RAG>(p, j) + c]);
+        else f[i] = Pop<S>::cvt(((const S *)(buf + j * SLOT))[lead<S, 1>(j) + c]);
     }
     R rho, ux, uy, uz;
     const R om0[3] = {0, 0, 0};
@@ -783,7 +779,7 @@ __device__ __forceinline__ void zwrap_cell(const LatParams &p, const StepParams 
     for (int i = 0; i < 19; i++) {
         const S v = Pop<S>::enc(f[i], rng);
         if (i > 0 && CZ(i) == zw) pop[(uint64_t)i * p.NP + (uint32_t)((int32_t)n + nb.off(CX(i), CY(i), CZ(i)))] = v;
-        else ((S *)(buf + i * SLOT))[lead_of<S, 1, RAG>(p, i) + c] = v;
+        else ((S *)(buf + i * SLOT))[lead<S, 1>(i) + c] = v;
     }
 }
 
@@ -794,8 +790,8 @@ __device__ __forceinline__ void zwrap_cell(const LatParams &p, const StepParams 
 // and direction where the plane's lead is even.  relax_fixed keeps every
 // rounding, and each cell draws the random bits it drew alone, so results are
 // the same.  us per step, one cell per thread -> pairs: 512x256x256 FP16 531 ->
-// 493, BF16 541 -> 490, 320x160x160 FP16 174 -> 145.  A fluid cell is never at the end of a row (x is not periodic), so
-// a pair that holds one lies in one row.
+// 493, BF16 541 -> 490, 320x160x160 FP16 174 -> 145.  A fluid cell is never at
+// the end of a row (x is not periodic), so a pair that holds one lies in one row.
 template <class S> __device__ __forceinline__ F2 pair_floats(uint32_t w);
 template <> __device__ __forceinline__ F2 pair_floats<__half>(uint32_t w) { return F2(__half22float2(*reinterpret_cast<const __half2 *>(&w))); }
 template <> __device__ __forceinline__ F2 pair_floats<__nv_bfloat16>(uint32_t w) {
@@ -819,10 +815,12 @@ __device__ __forceinline__ void bulk_pairs(const LatParams &p, const StepParams 
         uint32_t x, y, z;
         coords(p, a0 ? n : n + 1, x, y, z);
         if (!a0) x--;  // (the row of the fluid cell; it is not the row's first)
-        if (P == 1 && zper && (z == 0 || z == p.NZ - 1)) {
-            if (a0) zwrap_cell<S, 0, RAG>(p, s, buf, c, n, x, y, z);
-            if (a1) zwrap_cell<S, 0, RAG>(p, s, buf, c + 1, n + 1, x + 1, y, z);
-            continue;
+        if constexpr (P == 1 && !RAG) {
+            if (zper && (z == 0 || z == p.NZ - 1)) {
+                if (a0) zwrap_cell<S, 0>(p, s, buf, c, n, x, y, z);
+                if (a1) zwrap_cell<S, 0>(p, s, buf, c + 1, n + 1, x + 1, y, z);
+                continue;
+            }
         }
         F2 f[19];
 #pragma unroll
@@ -893,18 +891,19 @@ __device__ __forceinline__ void bulk_pairs(const LatParams &p, const StepParams 
 #pragma unroll
             for (int i = 0; i < 19; i++) dst(i)[1] = Pop<S>::bits(out[i] >> 16);
         }
-        if ((fg.x | fg.y) & FLAG_XFACE) {
+        if constexpr (!RAG) {
+            if (!((fg.x | fg.y) & FLAG_XFACE)) continue;
             // (only fluid cells carry the bit; a row of four has both its cells in one pair)
             S o[19];
             if (a0 && (fg.x & FLAG_XFACE)) {
 #pragma unroll
                 for (int i = 0; i < 19; i++) o[i] = Pop<S>::bits(out[i] & 0xffffu);
-                xface_from_inner<S, P, RAG>(p, s, buf, c, n, x, y, z, o);
+                xface_from_inner<S, P>(p, s, buf, c, n, x, y, z, o);
             }
             if (a1 && (fg.y & FLAG_XFACE)) {
 #pragma unroll
                 for (int i = 0; i < 19; i++) o[i] = Pop<S>::bits(out[i] >> 16);
-                xface_from_inner<S, P, RAG>(p, s, buf, c + 1, n + 1, x + 1, y, z, o);
+                xface_from_inner<S, P>(p, s, buf, c + 1, n + 1, x + 1, y, z, o);
             }
         }
     }
@@ -1023,9 +1022,11 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
             if ((fg & ~FLAG_XFACE) != 0u) continue;
             uint32_t x, y, z;
             coords(p, n, x, y, z);
-            if (P == 1 && zper && (z == 0 || z == p.NZ - 1)) {
-                zwrap_cell<S, COLL, RAG>(p, s, buf, c, n, x, y, z);
-                continue;
+            if constexpr (P == 1 && !RAG) {
+                if (zper && (z == 0 || z == p.NZ - 1)) {
+                    zwrap_cell<S, COLL>(p, s, buf, c, n, x, y, z);
+                    continue;
+                }
             }
             // FP16 values stay in storage units (x 32768) through the collision
             constexpr int SC = std::is_same<S, __half>::value ? (int)FP16_SCALE : 1;
@@ -1037,7 +1038,8 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
                 if constexpr (SC != 1) f[i] = __half2float(v);
                 else f[i] = Pop<S>::cvt(v);
             }
-            if constexpr (RAG && FEAT != 0 && COLL == 0 && sizeof(R) == 4) {
+            if constexpr (RAG) {
+                static_assert(FEAT != 0 && COLL == 0 && sizeof(R) == 4, "the forms that ragged rows are staged with");
                 // the direct kernel's roundings (its lattices' results stay
                 // what they were before they were staged)
                 const R sp = p.sponge_on ? sponge_at<R>(k, p, x, y, z) : (R)0;
@@ -1072,7 +1074,9 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
                 const int j = (P == 0) ? OPP(i) : i;  // plane receiving output f[i]
                 ((S *)(buf + j * SLOT))[lead_of<S, P, RAG>(p, j) + c] = out[i];
             }
-            if (fg & FLAG_XFACE) xface_from_inner<S, P, RAG>(p, s, buf, c, n, x, y, z, out);
+            if constexpr (!RAG) {
+                if (fg & FLAG_XFACE) xface_from_inner<S, P>(p, s, buf, c, n, x, y, z, out);
+            }
         }
         fence_async_smem();  // this thread's shared-memory writes, before the bulk stores read them
         mbar_arrive(&empty[b]);
@@ -1449,9 +1453,9 @@ static unsigned tma_grid() {
 template <class S, int P, int COLL, int FEAT>
 static void launch_tma(const LatParams &p, const StepParams &s, cudaStream_t st, bool pdl) {
     const unsigned ntiles = (unsigned)((p.N + Tile<S>::cells - 1) / Tile<S>::cells);
-    // (ragged FP32, FP16 and BF16 lattices come here only with the regularized
-    // collision and compile-time features)
-    if constexpr (sizeof(S) == 8 || (COLL == 0 && FEAT != 0)) {
+    // (ragged lattices come here only with the regularized collision in FP32 and
+    // compile-time features)
+    if constexpr (sizeof(S) != 8 && COLL == 0 && FEAT != 0) {
         if (p.ragged) {
             launch_pdl(pdl, k_bulk_tma<S, P, COLL, FEAT, true>, std::min(ntiles, tma_grid<S, P, COLL, FEAT, true>()), Tma<S>::threads, tma_smem<S>(), st, p, s);
             return;
