@@ -704,8 +704,10 @@ void run_impl(lbm_lattice *h, const lbm_step_in *steps, uint64_t n, double *forc
             h->steps_done++;
             h->scr ^= 1u;
             h->fused_valid = h->xfuse;
-            if (p.nrec && ((k + 1) % h->ring == 0 || k + 1 == len))
+            if (p.nrec && ((k + 1) % h->ring == 0 || k + 1 == len)) {
                 ck(lbm::launch_force_sum(p, k - k % h->ring, k % h->ring + 1, h->stream), "force sum");
+                if (h->prof) h->prof_launches++;
+            }
         }
         if (readback) {
             ck(cudaMemcpyAsync(h->hist_host, p.hist, len * 8 * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "history readback");
