@@ -787,12 +787,13 @@ __global__ void __launch_bounds__(BLK) k27_dump(const __grid_constant__ LevelPar
                             (float)(mo.j[2] / rho - (R)0.5 * k.grav[2]));
 }
 
-// Density and velocity of a cell of a level between steps, from its current
-// source set (mshader.rs:495-505): every cell type but solid has them.
+// Density and velocity of an updated fluid cell of a level between steps, from
+// its current source set (mshader.rs:495-505).  Face, ghost and restricted cells
+// have none: they store only the directions that are read from them.
 template <class S>
 __device__ __forceinline__ bool cell_macro27(const LevelParams &p, uint32_t src, uint32_t n, float &rho, float &ux, float &uy, float &uz) {
     using R = typename Pop<S>::real;
-    if ((p.flags[n] & 7u) == T_SOLID) return false;
+    if ((p.flags[n] & 7u) != 0) return false;
     const Consts27<R> &k = K<R>(p);
     R f[27];
     own<S>(p, src, n, f);
