@@ -789,7 +789,8 @@ __device__ __forceinline__ void zwrap_cell(const LatParams &p, const StepParams 
 // through the packed arithmetic of f32x2.cuh, one shared-memory word per plane
 // and direction where the plane's lead is even.  relax_fixed keeps every
 // rounding, and each cell draws the random bits it drew alone, so results are
-// the same.  us per step, one cell per thread -> pairs: 512x256x256 FP16 531 ->
+// the same (SIMLAB_LBM_ONE_CELL=1 keeps one cell per thread, to compare with).
+// us per step, one cell per thread -> pairs: 512x256x256 FP16 531 ->
 // 493, BF16 541 -> 490, 320x160x160 FP16 174 -> 145.  A fluid cell is never at
 // the end of a row (x is not periodic), so a pair that holds one lies in one row.
 template <class S> __device__ __forceinline__ F2 pair_floats(uint32_t w);
@@ -909,7 +910,10 @@ __device__ __forceinline__ void bulk_pairs(const LatParams &p, const StepParams 
     }
 }
 
-template <class S, int P, int COLL, int FEAT, bool RAG>
+// the forms that take two cells per thread
+template <class S, int COLL, int FEAT> constexpr bool in_pairs() { return sizeof(S) == 2 && COLL == 0 && FEAT != 0; }
+
+template <class S, int P, int COLL, int FEAT, bool RAG, bool PAIRS = in_pairs<S, COLL, FEAT>()>
 __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tma(const __grid_constant__ LatParams p, const __grid_constant__ StepParams s) {
     using R = typename Pop<S>::real;
     constexpr int NBUF = Nbuf<S>::value;
@@ -1011,7 +1015,7 @@ __global__ void __launch_bounds__(Tma<S>::threads, Tma<S>::min_blocks) k_bulk_tm
         uint8_t *buf = sm + b * BUF;
         const uint32_t *fl = (const uint32_t *)(buf + 19 * SLOT);
         const uint32_t n0 = tile_start<P>(t, ntiles, T);
-        if constexpr (sizeof(S) == 2 && COLL == 0 && FEAT != 0) {
+        if constexpr (PAIRS) {
             bulk_pairs<S, P, FEAT, RAG>(p, s, buf, n0, zper);
         } else
 #pragma unroll 1
@@ -1436,11 +1440,11 @@ static int num_sms() {
 }
 
 // persistent grid of the staged kernel: resident blocks per SM x SMs
-template <class S, int P, int COLL, int FEAT, bool RAG>
+template <class S, int P, int COLL, int FEAT, bool RAG, bool PAIRS>
 static unsigned tma_grid() {
     static unsigned g = 0;
     if (!g) {
-        auto kern = k_bulk_tma<S, P, COLL, FEAT, RAG>;
+        auto kern = k_bulk_tma<S, P, COLL, FEAT, RAG, PAIRS>;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tma_smem<S>());
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Tma<S>::threads, tma_smem<S>());
@@ -1453,15 +1457,21 @@ static unsigned tma_grid() {
 template <class S, int P, int COLL, int FEAT>
 static void launch_tma(const LatParams &p, const StepParams &s, cudaStream_t st, bool pdl) {
     const unsigned ntiles = (unsigned)((p.N + Tile<S>::cells - 1) / Tile<S>::cells);
+    auto go = [&](auto rag, auto pairs) {
+        constexpr bool RAG = decltype(rag)::value, PAIRS = decltype(pairs)::value;
+        launch_pdl(pdl, k_bulk_tma<S, P, COLL, FEAT, RAG, PAIRS>, std::min(ntiles, tma_grid<S, P, COLL, FEAT, RAG, PAIRS>()), Tma<S>::threads,
+                   tma_smem<S>(), st, p, s);
+    };
+    constexpr std::bool_constant<in_pairs<S, COLL, FEAT>()> pairs{};
     // (ragged lattices come here only with the regularized collision in FP32 and
     // compile-time features)
     if constexpr (sizeof(S) != 8 && COLL == 0 && FEAT != 0) {
-        if (p.ragged) {
-            launch_pdl(pdl, k_bulk_tma<S, P, COLL, FEAT, true>, std::min(ntiles, tma_grid<S, P, COLL, FEAT, true>()), Tma<S>::threads, tma_smem<S>(), st, p, s);
-            return;
-        }
+        if (p.ragged) return go(std::true_type{}, pairs);
     }
-    launch_pdl(pdl, k_bulk_tma<S, P, COLL, FEAT, false>, std::min(ntiles, tma_grid<S, P, COLL, FEAT, false>()), Tma<S>::threads, tma_smem<S>(), st, p, s);
+    if constexpr (pairs) {
+        if (p.one_cell) return go(std::false_type{}, std::false_type{});
+    }
+    go(std::false_type{}, pairs);
 }
 
 // One step: faces and wall cells, then the bulk.  Where no wall cell is near a

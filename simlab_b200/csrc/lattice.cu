@@ -552,6 +552,8 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
     // units take its variant with the planes' misalignments as parameters
     p.tma = tma_ok;
     p.ragged = ragged;
+    const char *one_cell = std::getenv("SIMLAB_LBM_ONE_CELL");
+    p.one_cell = one_cell && one_cell[0] == '1';
     for (int j = 0; j < 19; j++) {
         const int64_t unit = (int64_t)(16 / sb);
         const int64_t shift = lbm::CX(j) + lbm::CY(j) * (int64_t)NX + lbm::CZ(j) * (int64_t)(NX * NY);

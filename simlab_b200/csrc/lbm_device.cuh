@@ -148,6 +148,7 @@ struct LatParams {
     FastDiv frect_nu[6];
     int tma;                   // the staged bulk kernel applies (x and y not periodic)
     int ragged;                // its rows are no whole number of 16-byte units
+    int one_cell;              // one cell per thread where it would take two (aligned rows)
     // ragged rows, parity 1: elements by which plane j's slots miss a 16-byte
     // boundary at an aligned cell (c_j's shift modulo the unit)
     uint32_t lead[19];
