@@ -381,11 +381,15 @@ def plan(cfg: WindConfig, m: Mesh, unit_m: float, opt: SolverOptions, budget: Op
     est_records = int(np.prod(box_n)) if spin is not None else int(2.0 * area_m2 / (dx * dx)) + 1000
     faces_cells = 2 * (dims[0] * dims[1] + dims[1] * dims[2] + dims[0] * dims[2])
 
+    # a spinning part's re-voxelizer: two sets of 27 words of link scratch per
+    # box cell, and a byte per cell of the box and the layer around it
+    revoxel = est_records * 2 * 27 * 4 + int(np.prod(np.asarray(box_n) + 2)) if spin is not None else 0
+
     def mem_for(s: int) -> int:
         if multi is not None:
             pops = sum(c * (2 * 27 * _pop_bytes(s) + 4 + 8) for c in multi.cells)
             return pops + est_records * 24 * 4 * 2 + 64 * 1024 * 1024
-        return n * (19 * _pop_bytes(s) + 4) + est_records * 40 * 4 + faces_cells * 44 + 64 * 1024 * 1024
+        return n * (19 * _pop_bytes(s) + 4) + est_records * 40 * 4 + revoxel + faces_cells * 44 + 64 * 1024 * 1024
 
     n_max = max(multi.cells) if multi is not None else n
 
