@@ -409,10 +409,17 @@ struct lbm_gray {
     uint64_t nbox() const { return (uint64_t)p.box_n[0] * p.box_n[1] * p.box_n[2]; }
     size_t set_bytes() const { return (size_t)19 * p.NP * ssz; }   // a population set (or checkpoint)
     size_t lset_bytes() const { return (size_t)19 * p.NP * rsz; }  // an adjoint set
-    // Walk the lattice backwards every other step where two sets are at most 2.5
-    // times L2 (126 MB): the gradient of 192x96x96 FP32 (2 x 134 MB) 38.4 -> 36.7
-    // ms; of 384x192x192 FP16 (2 x 540 MB, the adjoint's twice that) 54 -> 58.
-    static bool backwards(size_t bytes) { return 2 * bytes <= (320ull << 20); }
+    // Walk the lattice backwards every other step where two sets are at most five
+    // times L2 (126 MB): the cells that L2 still holds are a smaller and smaller
+    // share of a larger lattice.  Forwards only -> in turn, by the bytes of two
+    // sets, ms per 100 forward steps: FP32 148 MB 3.54 -> 3.25, 256 5.84 -> 5.52, 326
+    // 6.87 -> 6.55, 407 8.70 -> 8.40, 608 12.51 -> 12.30; FP16 128 5.00 -> 4.82, 304
+    // 11.18 -> 11.08, 593 21.34 -> 21.25, 1026 36.40 -> 36.31.  The adjoint, by ms per
+    // gradient of 60 steps: 148 MB 5.15 -> 4.87, 256 8.59 -> 8.13, 407 12.75 -> 12.2,
+    // 608 19.3 -> 19.0, 865 24.6 -> 24.5, 1187 33.4 -> 33.2, 2052 55.4 -> 56.0 (FP32 sets
+    // of FP16 lattices from 865 on).
+    size_t l2 = 0;  // bytes, of the device the handle is on
+    bool backwards(size_t bytes) const { return 2 * bytes <= 5 * l2; }
     void *dalloc(size_t bytes) {
         void *q = nullptr;
         ck(cudaMalloc(&q, std::max<size_t>(bytes, 16)), "cudaMalloc");
@@ -712,6 +719,10 @@ void create_gray(const lbm_gray_setup *s, lbm_gray *h) {
     fill<float>(p.kf, *s);
     fill<double>(p.kd, *s);
     ck(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "cudaStreamCreate");
+    int dev = 0, l2 = 0;
+    ck(cudaGetDevice(&dev), "cudaGetDevice");
+    ck(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev), "cudaDeviceGetAttribute");
+    h->l2 = (size_t)l2;
     ck(cudaEventCreateWithFlags(&h->ev, cudaEventDisableTiming), "cudaEventCreate");
     h->P[0] = h->dalloc(h->set_bytes());
     h->P[1] = h->dalloc(h->set_bytes());
