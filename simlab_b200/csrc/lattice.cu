@@ -395,12 +395,14 @@ void create_impl(const lbm_setup *setup, const lbm_geometry *geom, const lbm_pro
     // regularized collision in FP32 without a body force, without the u_inf
     // absorbing target and without periodic z.  Small lattices stay with the
     // direct kernel too: the staged kernel's few large tiles leave SMs idle.
-    // Measured, us per step of a sphere in a tunnel, direct / staged: FP32 0.41 M
-    // cells 26.7 / 28.7, 0.82 M 36.0 / 36.8, 1.7 M 73.4 / 70.5, 3.6 M 134.6 /
-    // 122.3; FP16 28.2 / 31.3, 41.1 / 37.8, 67.0 / 52.0, 134.6 / 90.1 (BF16 like
+    // Measured, us per step of a sphere in a tunnel, direct / staged: 0.40 M cells
+    // FP32 20.5 / 20.4, FP16 22.1 / 22.8; 0.45 M 21.6 / 21.1, 23.1 / 23.4; 0.50 M
+    // 22.1 / 21.0, 24.7 / 23.9; 0.70 M 27.1 / 24.5, - / 24.1; 0.82 M 30.0 / 28.1, 33.5 /
+    // 29.2; 0.99 M 33.9 / 34.2 (the last round of tiles is nearly empty), - / 28.8;
+    // 1.7 M 57.3 / 50.5, 57.8 / 40.8; 3.1 M 106.7 / 93.8, 107.0 / 68.2 (BF16 like
     // FP16).  FP64 stays with it at every size: 27.6 / 27.6 at 0.1 M, 231 / 230 at
     // 3.6 M, for other roundings.
-    const uint64_t ragged_from = st.storage == LBM_STORAGE_FP32 ? 1000000 : 640000;
+    const uint64_t ragged_from = 500000;
     const bool tma_ok = !per[0] && !per[1] && !(no_tma && no_tma[0] == '1') &&
                         (!ragged || (st.storage != LBM_STORAGE_FP64 && N >= ragged_from && st.collision == LBM_COLLISION_REGULARIZED &&
                                      !force && !st.absorb_velocity && !per[2]));

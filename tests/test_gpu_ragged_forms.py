@@ -56,3 +56,10 @@ def test_every_form_above_the_size_of_the_staged_kernel(storage, form, monkeypat
 @pytest.mark.parametrize("form", ["les_sponge", "plain"])
 def test_two_byte_rows(storage, nx, form, monkeypatch):
     _check((nx, 66, 65), storage, form, monkeypatch)
+
+
+@pytest.mark.parametrize("storage", [Storage.FP32, Storage.FP16, Storage.BF16])
+@pytest.mark.parametrize("dims", [(125, 71, 57), (113, 67, 67), (1501, 19, 19)])  # about the smallest that are staged: 505,875, 507,257, 541,861 cells
+@pytest.mark.parametrize("form", ["les_sponge", "plain"])
+def test_smallest_staged(storage, dims, form, monkeypatch):
+    _check(dims, storage, form, monkeypatch)
