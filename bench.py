@@ -43,13 +43,16 @@ METRIC = "MLUPS (D3Q19 LES arm 512x256x256, FP16-stored populations)"
 UNIT = "MLUPS"
 DTYPE = "f32 arithmetic, fp16 storage"
 # Arithmetic per lattice update of the two collision kernels, FP16 storage,
-# from ncu's counters (profiles/opcode_mix_k_bulk_tma_k27_step_fp16.md):
+# from ncu's counters (profiles/pairs_ragged_k27_step_revoxel_walls_faces.md):
 # flops = FADD + FMUL + 2 FFMA thread instructions executed with the
-# predicate on, per cell; instructions = executed warp instructions x 32 per
-# cell (smsp__inst_executed; D3Q19 includes the copy pipeline's wait loops).  FP32 peak: 148 SMs x 128 FP32
-# lanes x 2 flops x clock; issue peak: 148 SMs x 4 schedulers x 32 threads x clock.
-ALU_PER_LUP = {"d3q19_bulk_fp16": {"flops": 78.93 + 40.80 + 2 * 63.71, "instr": 410.8},
-               "d3q27_step_fp16": {"flops": 163.76 + 82.50 + 2 * 135.74, "instr": 1012.4}}
+# predicate on, per cell (D3Q19: of the one-cell form, whose arithmetic the
+# packed instructions do two cells at a time); instructions = executed warp
+# instructions x 32 per cell, D3Q19 the mean of the two parities
+# (smsp__inst_executed; it includes the copy pipeline's wait loops).  FP32 peak:
+# 148 SMs x 128 FP32 lanes x 2 flops x clock; issue peak: 148 SMs x 4 schedulers
+# x 32 threads x clock.
+ALU_PER_LUP = {"d3q19_bulk_fp16": {"flops": 78.93 + 40.80 + 2 * 63.71, "instr": 308.1},
+               "d3q27_step_fp16": {"flops": 159.9 + 81.5 + 2 * 135.7, "instr": 994.0}}
 
 
 def alu_line(lups: dict, sm_mhz: float) -> dict:
@@ -58,7 +61,7 @@ def alu_line(lups: dict, sm_mhz: float) -> dict:
     f = sm_mhz * 1e6
     peak_fp32, peak_issue = 148 * 128 * 2 * f, 148 * 4 * 32 * f
     out = {"fp32_peak_tflops": round(peak_fp32 / 1e12, 2), "issue_peak_tinst_s": round(peak_issue / 1e12, 2), "sm_mhz": sm_mhz,
-           "source": "profiles/opcode_mix_k_bulk_tma_k27_step_fp16.md"}
+           "source": "profiles/pairs_ragged_k27_step_revoxel_walls_faces.md"}
     for k, ups in lups.items():
         c = ALU_PER_LUP[k]
         out[k] = {"flops_per_lup": round(c["flops"], 1), "instr_per_lup": c["instr"], "glups": round(ups / 1e9, 2),
